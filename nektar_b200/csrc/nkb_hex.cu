@@ -359,6 +359,8 @@ static bool SameTable(const std::vector<double> &a, const std::vector<double> &b
 int ChooseKernel(nkb_op *op)
 {
     op->variant  = kVariantGeneric;
+    if (!op->line_tabs.empty())
+        return NKB_OK; // a line kernel (nkb_line.cu): nothing to choose
     const int eb = op->precision == NKB_FP64 ? 8 : 4;
     if (op->shape == NKB_HEX && (op->optype == NKB_HELMHOLTZ || op->optype == NKB_LINEAR_ADR) &&
         op->nm >= 2 && op->nm <= 11 &&
@@ -465,14 +467,10 @@ const char *KernelName(const nkb_op *op, bool gather)
         return "k_dense_gemv (per-element dense blocks)";
     if (op->variant != kVariantHexHelm)
     {
-        const int nm   = op->nm;
-        const bool std = op->nq[0] == nm + 1 &&
-                         ((op->shape == NKB_PRISM && op->nq[1] == nm + 1 && op->nq[2] == nm) ||
-                          (op->shape == NKB_TET && op->nq[1] == nm && op->nq[2] == nm));
-        if ((op->optype == NKB_HELMHOLTZ || op->optype == NKB_LINEAR_ADR) && std && nm >= 2 &&
-            nm <= 11)
-            return "k_col_helm (Prism/Tet column kernel)";
-        return "k_generic";
+        const bool helm = op->optype == NKB_HELMHOLTZ || op->optype == NKB_LINEAR_ADR;
+        if (helm && op->shape != NKB_HEX && !op->line_tabs.empty())
+            return "k_col_helm (Prism/Tet column kernel: k_line)";
+        return op->line_tabs.empty() ? "k_generic" : "k_line (one thread per grid line)";
     }
     const int v = (gather && op->hex_variant_gather >= 0) ? op->hex_variant_gather : op->hex_variant;
     switch (v)

@@ -35,6 +35,13 @@ struct nkb_op
     int diff_mode    = NKB_DIFF_NONE;
     double diff[6]   = {1, 0, 1, 0, 0, 1};
 
+    // line kernels (nkb_line.cu): their tables in parameter layout (empty: not
+    // used); packed geometry with the third direction fastest; 16 values per
+    // straight-sided element
+    std::vector<unsigned char> line_tabs;
+    int geo_perm = 0;
+    double *geoc = nullptr;
+
     // kernel selection (nkb_hex.cu): 0 generic, >0 tuned variant
     int variant     = 0;
     int hex_variant = 0; // tuned Hex kernel variant chosen by the autotuner
@@ -70,6 +77,13 @@ template <typename T>
 int LaunchGeneric3(const nkb_op *op, const T *in, const T *in1, const T *in2, T *o0, T *o1, T *o2,
                    const int *gmap, const double *gsign, cudaStream_t s,
                    const int *skip = nullptr, const double *lambda = nullptr);
+// line kernels (nkb_line.cu). LineSetup decides whether the operator runs on
+// them and prepares its tables and layout (before the geometry is packed);
+// LaunchLine launches the one that was set up
+int LineSetup(nkb_op *op);
+template <typename T>
+int LaunchLine(const nkb_op *op, const T *in, const T *in1, const T *in2, T *o0, T *o1, T *o2,
+               const int *gmap, const double *gsign, cudaStream_t s, const int *skip, T lambda);
 // per-element dense operators (nkb_dense.cu)
 int LaunchDense(const nkb_op *op, const double *in, double *out, const int *gmap,
                 const double *gsign, cudaStream_t s, const int *skip);

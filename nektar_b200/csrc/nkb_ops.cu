@@ -104,7 +104,68 @@ struct PackArgs
     int ncomp;                    // 7 Helmholtz, 10 LinearADR, 9 PhysDeriv /
                                   // IProductWRTDerivBase, 1 IProduct
     long gstride;                 // element stride of the packed arrays
+    int perm;                     // points packed with the third direction fastest
+    double *geoc;                 // straight-sided elements: 16 values per element
+                                  // (nkb_line_kernel.cuh)
 };
+
+// the diffusion tensor of the operator's mode
+__device__ void DiffusionTensor(const PackArgs &a, double K[3][3])
+{
+    for (int x = 0; x < 3; ++x)
+        for (int y = 0; y < 3; ++y)
+            K[x][y] = x == y ? 1.0 : 0.0;
+    if (a.diff_mode == NKB_DIFF_NONE)
+        return;
+    K[0][0] = a.K[0];
+    K[0][1] = K[1][0] = a.K[1];
+    K[1][1]           = a.K[2];
+    K[0][2] = K[2][0] = a.K[3];
+    K[1][2] = K[2][1] = a.K[4];
+    K[2][2]           = a.K[5];
+    // the reference Tet kernel keeps d11 = 1 under variable diffusion
+    // (HelmholtzKernels.hpp:453-460 never loads varD11)
+    if (a.shape == NKB_TET && a.diff_mode == NKB_DIFF_VAR)
+        K[1][1] = 1.0;
+}
+
+// Straight-sided elements: Jacobian, J F K F^T and the derivative factors F
+// (F[k*3+j] = d xi_j / d x_k) once per element. The line kernels multiply in
+// the weights and collapsed-coordinate factors, which are products of 1-D tables.
+__global__ void k_pack_straight(PackArgs a)
+{
+    for (long e = blockIdx.x * long(blockDim.x) + threadIdx.x; e < a.nelmt;
+         e += long(gridDim.x) * blockDim.x)
+    {
+        double v[16];
+        for (int c = 0; c < 16; ++c)
+            v[c] = 0.0;
+        v[0] = a.jac ? a.jac[e] : 1.0;
+        if (a.df)
+        {
+            double K[3][3];
+            DiffusionTensor(a, K);
+            double *F = v + 7;
+            for (int d = 0; d < 9; ++d)
+                F[d] = a.df[d * long(a.nelmt) + e];
+            auto metric = [&](int x, int y) {
+                double s = 0.0;
+                for (int k = 0; k < 3; ++k)
+                    for (int l = 0; l < 3; ++l)
+                        s += F[k * 3 + x] * K[k][l] * F[l * 3 + y];
+                return v[0] * s;
+            };
+            v[1] = metric(0, 0);
+            v[2] = metric(1, 1);
+            v[3] = metric(2, 2);
+            v[4] = metric(0, 1);
+            v[5] = metric(0, 2);
+            v[6] = metric(1, 2);
+        }
+        for (int c = 0; c < 16; ++c)
+            a.geoc[e * 16 + c] = v[c];
+    }
+}
 
 __global__ void k_scale(double *v, size_t n, double s)
 {
@@ -125,8 +186,9 @@ __global__ void k_pack(PackArgs a)
         const long ncol = a.deformed ? tot : long(a.nelmt);
         const long col  = a.deformed ? g : e;
         const double J  = a.jac ? a.jac[col] : 1.0;
-        double *out     = a.geo + e * a.gstride + q;
-        float *out32    = a.geo32 ? a.geo32 + e * a.gstride + q : nullptr;
+        const long at   = e * a.gstride + (a.perm ? (long(i) * a.nq1 + j) * a.nq2 + k : q);
+        double *out     = a.geo + at;
+        float *out32    = a.geo32 ? a.geo32 + at : nullptr;
         if (a.optype == NKB_IPRODUCT)
         {
             double W = J * a.w0[i] * a.w1[j] * a.w2[k];
@@ -154,20 +216,8 @@ __global__ void k_pack(PackArgs a)
             continue;
         }
         // Helmholtz: W and W * A K A^T (six unique entries)
-        double K[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
-        if (a.diff_mode != NKB_DIFF_NONE)
-        {
-            K[0][0] = a.K[0];
-            K[0][1] = K[1][0] = a.K[1];
-            K[1][1]           = a.K[2];
-            K[0][2] = K[2][0] = a.K[3];
-            K[1][2] = K[2][1] = a.K[4];
-            K[2][2]           = a.K[5];
-            // the reference Tet kernel keeps d11 = 1 under variable diffusion
-            // (HelmholtzKernels.hpp:453-460 never loads varD11)
-            if (a.shape == NKB_TET && a.diff_mode == NKB_DIFF_VAR)
-                K[1][1] = 1.0;
-        }
+        double K[3][3];
+        DiffusionTensor(a, K);
         double t[3][3];
         for (int x = 0; x < 3; ++x)
             for (int l = 0; l < 3; ++l)
@@ -211,8 +261,9 @@ static Dims MakeDims(const nkb_op *op);
 
 // Diagonal of the element Helmholtz matrix: for every mode m,
 // diag_m = sum_q lambda W phi_m^2 + grad phi_m . G' grad phi_m,
-// phi_m = BwdTrans(e_m). One CTA per element.
-template <int SHAPE, typename T> __global__ void k_diag(GenArgs<T> a)
+// phi_m = BwdTrans(e_m). One CTA per element. perm: the geometry's points lie
+// with the third direction fastest.
+template <int SHAPE, typename T> __global__ void k_diag(GenArgs<T> a, int perm)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *smem       = reinterpret_cast<T *>(smem_raw);
@@ -243,8 +294,10 @@ template <int SHAPE, typename T> __global__ void k_diag(GenArgs<T> a)
         {
             T q0, q1, q2;
             Grad(d, a.t, u, l, q0, q1, q2);
-            const T W = G[l], G00 = G[d.nt + l], G11 = G[2 * d.nt + l], G22 = G[3 * d.nt + l];
-            const T G01 = G[4 * d.nt + l], G02 = G[5 * d.nt + l], G12 = G[6 * d.nt + l];
+            const int i = l % d.nq0, j = (l / d.nq0) % d.nq1, k = l / (d.nq0 * d.nq1);
+            const int g = perm ? (i * d.nq1 + j) * d.nq2 + k : l;
+            const T W = G[g], G00 = G[d.nt + g], G11 = G[2 * d.nt + g], G22 = G[3 * d.nt + g];
+            const T G01 = G[4 * d.nt + g], G02 = G[5 * d.nt + g], G12 = G[6 * d.nt + g];
             T v = q0 * fma(G00, q0, 2 * (G01 * q1 + G02 * q2));
             v   = fma(q1, fma(G11, q1, 2 * G12 * q2), v);
             v   = fma(q2, G22 * q2, v);
@@ -416,21 +469,11 @@ template <int OP, typename T> static int LaunchGenericShape(const nkb_op *op, Ge
 }
 
 extern template int LaunchHelmStatic<double>(const nkb_op *, const GenArgs<double> &, cudaStream_t);
-// Prism / Tet column kernels (nkb_col_kernel.cuh, nkb_col_f64.cu, nkb_col_f32.cu)
-template <typename T> int LaunchColHelm(const nkb_op *op, const GenArgs<T> &a, cudaStream_t s);
-extern template int LaunchColHelm<double>(const nkb_op *, const GenArgs<double> &, cudaStream_t);
-extern template int LaunchColHelm<float>(const nkb_op *, const GenArgs<float> &, cudaStream_t);
 extern template int LaunchHelmStatic<float>(const nkb_op *, const GenArgs<float> &, cudaStream_t);
 
 static bool StaticSizes()
 {
     const char *v = std::getenv("NKB_GENERIC_STATIC");
-    return !(v && std::strcmp(v, "0") == 0);
-}
-
-static bool ColKernels()
-{
-    const char *v = std::getenv("NKB_COL");
     return !(v && std::strcmp(v, "0") == 0);
 }
 
@@ -450,6 +493,9 @@ int LaunchGeneric3(const nkb_op *op, const T *in, const T *in1, const T *in2, T 
                    const int *gmap, const double *gsign, cudaStream_t s, const int *skip,
                    const double *lambda)
 {
+    if (!op->line_tabs.empty())
+        return LaunchLine<T>(op, in, in1, in2, o0, o1, o2, gmap, gsign, s, skip,
+                             T(lambda ? *lambda : op->lambda));
     GenArgs<T> a;
     a.d      = MakeDims(op);
     a.t      = MakeTabs<T>(op);
@@ -478,21 +524,9 @@ int LaunchGeneric3(const nkb_op *op, const T *in, const T *in1, const T *in2, T 
         case NKB_IPRODUCT_DERIV:
             return LaunchGenericShape<GK_IPD, T>(op, a, s);
         case NKB_LINEAR_ADR:
-            if (ColKernels() && !gmap)
-            {
-                const int rc = LaunchColHelm<T>(op, a, s);
-                if (rc != kNotCovered)
-                    return rc;
-            }
             return LaunchGenericShape<GK_ADR, T>(op, a, s);
         default:
         {
-            if (ColKernels())
-            {
-                const int rc = LaunchColHelm<T>(op, a, s);
-                if (rc != kNotCovered)
-                    return rc;
-            }
             if (StaticSizes())
             {
                 const int rc = LaunchHelmStatic<T>(op, a, s);
@@ -545,11 +579,18 @@ static int Repack(nkb_op *op)
     a.geo32   = op->geo32;
     a.ncomp   = op->ncomp;
     a.gstride = op->gstride;
+    a.perm    = op->geo_perm;
+    a.geoc    = op->geoc;
     if (op->ncomp == 0)
         return NKB_OK;
-    long tot = long(op->nelmt) * op->nt;
-    int nb   = int(std::min<long>((tot + 255) / 256, 148L * 16));
-    k_pack<<<std::max(nb, 1), 256, 0, op->stream>>>(a);
+    if (op->geo)
+    {
+        const long tot = long(op->nelmt) * op->nt;
+        const int nb   = int(std::min<long>((tot + 255) / 256, 148L * 16));
+        k_pack<<<std::max(nb, 1), 256, 0, op->stream>>>(a);
+    }
+    if (op->geoc)
+        k_pack_straight<<<(op->nelmt + 127) / 128, 128, 0, op->stream>>>(a);
     NKB_CUDA_TRY(cudaGetLastError());
     NKB_CUDA_TRY(cudaStreamSynchronize(op->stream));
     return NKB_OK;
@@ -733,12 +774,20 @@ extern "C" int nkb_op_create(const nkb_op_desc *desc, nkb_op **out)
     if (desc->df && op->ncomp > 1 && op->nelmt)
         if ((rc = Upload(&op->ddf, desc->df, size_t(9) * ncol)))
             return fail(rc);
+    if ((rc = LineSetup(op)))
+        return fail(rc);
     if (op->ncomp && op->nelmt)
     {
-        const size_t n = size_t(op->nelmt) * op->gstride;
-        if (cudaMalloc(&op->geo, n * sizeof(double)) != cudaSuccess)
+        const bool straight = !op->line_tabs.empty() && !op->deformed;
+        const size_t nc16   = size_t(op->nelmt) * 16;
+        if (straight && cudaMalloc(&op->geoc, nc16 * sizeof(double)) != cudaSuccess)
+            return fail(SetError(NKB_ERR_NOMEM, "nkb_op_create: geometry (%zu doubles)", nc16));
+        // values per point: straight-sided elements on the line kernels need
+        // them only for LinearADR's velocities and Helmholtz's diagonal
+        const size_t n = straight && !helm_like ? 0 : size_t(op->nelmt) * op->gstride;
+        if (n && cudaMalloc(&op->geo, n * sizeof(double)) != cudaSuccess)
             return fail(SetError(NKB_ERR_NOMEM, "nkb_op_create: geometry (%zu doubles)", n));
-        if (op->precision == NKB_FP32 && cudaMalloc(&op->geo32, n * sizeof(float)) != cudaSuccess)
+        if (n && op->precision == NKB_FP32 && cudaMalloc(&op->geo32, n * sizeof(float)) != cudaSuccess)
             return fail(SetError(NKB_ERR_NOMEM, "nkb_op_create: FP32 geometry"));
         if ((rc = Repack(op)))
             return fail(rc);
@@ -1171,12 +1220,12 @@ int HelmholtzDiag(const nkb_op *op, double *d_out, cudaStream_t s, double *d_sti
     a.skip          = nullptr;
     const int threads = 128;
     size_t smem = size_t(a.d.nc + a.d.nt + 2 * a.d.wsz + 2 * threads) * sizeof(double);
-    void (*kern)(GenArgs<double>) = op->shape == NKB_HEX     ? k_diag<NKB_HEX, double>
+    void (*kern)(GenArgs<double>, int) = op->shape == NKB_HEX     ? k_diag<NKB_HEX, double>
                                     : op->shape == NKB_PRISM ? k_diag<NKB_PRISM, double>
                                                              : k_diag<NKB_TET, double>;
     NKB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     if (op->nelmt > 0)
-        kern<<<op->nelmt, threads, smem, s>>>(a);
+        kern<<<op->nelmt, threads, smem, s>>>(a, op->geo_perm);
     NKB_CUDA_TRY(cudaGetLastError());
     return NKB_OK;
 }
@@ -1229,6 +1278,7 @@ extern "C" void nkb_op_destroy(nkb_op *op)
     cudaFree(op->dvel);
     cudaFree(op->geo);
     cudaFree(op->geo32);
+    cudaFree(op->geoc);
     cudaFree(op->scratch);
     cudaFree(op->d_err);
     cudaFree(op->tc_tab);

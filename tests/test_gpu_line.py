@@ -1,0 +1,99 @@
+"""The line kernels (nkb_line_kernel.cuh) against the shape-generic kernels:
+every operator on every shape, at the smallest and largest orders, point counts
+whose shared-memory rows are rotated (4 and 8) and not, over-integration,
+straight-sided and curved geometry, and element counts that leave the last CTA
+partly filled."""
+import numpy as np
+import pytest
+
+import nektar_b200 as nb
+from tests.helpers import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+OPS = ("bwdtrans", "iproduct", "physderiv", "iproduct_deriv", "helmholtz", "linear_adr")
+# two summation orders of the same sums: a few hundred roundings of 1.1e-16 (6e-8)
+# that add up as a random walk, times the operators' cancellation (about 10)
+TOL = {"fp64": 1e-13, "fp32": 5e-6}
+# (modes, points in the first direction)
+SIZES = [(2, 3), (3, 4), (4, 5), (6, 7), (7, 8), (8, 9), (9, 10), (11, 12), (2, 4), (3, 6), (4, 8),
+         (6, 8), (7, 11), (10, 12)]
+
+
+def _apply(op, x, dtype):
+    import torch
+    nout = 3 if op.optype == nb.PHYSDERIV else 1
+    xd = torch.tensor(x, dtype=dtype, device="cuda")
+    out = torch.full((nout, op.out_size), float("nan"), dtype=dtype, device="cuda")
+    op.apply_device(xd.data_ptr(), *[o.data_ptr() for o in out],
+                    stream=torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    return out.double().cpu().numpy().ravel()
+
+
+def _operator(name, mesh, precision, rng):
+    op = nb.Operator(name, mesh, precision=precision)
+    if name == "helmholtz":
+        op.set_factors(0.7, nb.DIFF_CONST, [1.5, 0.2, 0.8, -0.1, 0.3, 1.1])
+    if name == "linear_adr":
+        op.set_factors(0.7)
+        op.set_varcoeffs(*rng.uniform(-1, 1, (3, mesh.nelmt * mesh.nt)))
+    return op
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("amp", [0.05, 0.0])
+@pytest.mark.parametrize("nm,nq", SIZES)
+@pytest.mark.parametrize("shape", ["hex", "prism", "tet"])
+def test_line_and_generic_kernels_agree(monkeypatch, shape, nm, nq, amp, precision):
+    import torch
+    dtype = torch.float64 if precision == "fp64" else torch.float32
+    for n in ([1, 3] if nm < 9 else [1]):
+        m = nb.BoxMesh(shape, n, nm, nq, amp=amp)
+        for name in OPS:
+            line = _operator(name, m, precision, np.random.default_rng(nm))
+            monkeypatch.setenv("NKB_KERNEL", "generic")
+            generic = _operator(name, m, precision, np.random.default_rng(nm))
+            monkeypatch.delenv("NKB_KERNEL")
+            assert generic.kernel() == "k_generic"
+            x = np.random.default_rng(nq).uniform(-1, 1, line.in_size)
+            y, z = _apply(line, x, dtype), _apply(generic, x, dtype)
+            assert rel_l2(y, z) < TOL[precision], (name, n, line.kernel())
+
+
+@pytest.mark.parametrize("shape", ["prism", "tet"])
+@pytest.mark.parametrize("amp", [0.05, 0.0])
+def test_line_kernel_diagonal_and_gather(monkeypatch, shape, amp):
+    """The Helmholtz diagonal reads the line kernels' point order; a gathered
+    launch with signs, through the CG of a block-diagonal system."""
+    m = nb.BoxMesh(shape, 2, 5, 6, amp=amp)
+    op = _operator("helmholtz", m, "fp64", None)
+    nloc = m.nelmt * m.nc
+    rng = np.random.default_rng(6)
+    gmap = rng.permutation(nloc).astype(np.int32)
+    sign = rng.choice([-1.0, 1.0], nloc)
+    b = rng.uniform(-1, 1, nloc)
+    monkeypatch.setenv("NKB_KERNEL", "generic")
+    ref = _operator("helmholtz", m, "fp64", None)
+    monkeypatch.delenv("NKB_KERNEL")
+    assert rel_l2(op.helmholtz_diag(), ref.helmholtz_diag()) < 1e-13
+    xs = [nb.GlobalLinSys([o], gmap, nloc, 0, sign=sign).solve(b, tol=1e-13)[0] for o in (op, ref)]
+    assert rel_l2(*xs) < 1e-10
+
+
+def test_line_kernel_three_input_fields_and_infinities():
+    """IProductWRTDerivBase from three device arrays, and a value that is not
+    finite, which must stay in its own element."""
+    import torch
+    m = nb.BoxMesh("tet", 2, 4, 5)
+    op = nb.Operator("iproduct_deriv", m)
+    f = torch.rand(3, m.nelmt * m.nt, dtype=torch.float64, device="cuda")
+    f[1, 5 * m.nt + 3] = float("inf")
+    y, z = (torch.empty(op.out_size, dtype=torch.float64, device="cuda") for _ in range(2))
+    s = torch.cuda.current_stream().cuda_stream
+    parts = [v.clone() for v in f]
+    op.apply3_device(*[v.data_ptr() for v in parts], y.data_ptr(), stream=s)
+    op.apply_device(f.data_ptr(), z.data_ptr(), stream=s)
+    bad = ~torch.isfinite(y.view(m.nelmt, m.nc)).all(1)
+    assert torch.equal(y.view(torch.int64), z.view(torch.int64))
+    assert bad.nonzero().ravel().tolist() == [5]
