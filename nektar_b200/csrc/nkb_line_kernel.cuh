@@ -193,10 +193,12 @@ template <int SHAPE, int NM, int NQ, int OP, typename T> struct LineDims
     }
     static constexpr int EPB = Epb();
     static constexpr int TH  = (EPB * LMAX + 31) / 32 * 32;
-    // register budget per thread; the FP64 arrays held across barriers are
-    // three lines of K0 values
-    static constexpr int REGS = sizeof(T) == 8 ? (K0 <= 6 ? 96 : (K0 <= 8 ? 128 : 168))
-                                               : (K0 <= 8 ? 64 : (K0 <= 10 ? 96 : 128));
+    // register budget per thread: the lowest that spills (next to) nothing. Warps
+    // in flight hide the barriers and the shared-memory latency: at 80 instead of
+    // 128 registers the FP64 Helmholtz operator took 87 instead of 118 us (hex, 8
+    // modes x 7140), 103 instead of 143 (9 x 5172), 115 instead of 184 (tet, 8 x
+    // 10241); FP32 at 48 instead of 64 gained 0-25 %
+        static constexpr int REGS = sizeof(T) == 8 ? (K0 <= 10 ? 80 : 96) : (K0 <= 9 ? 48 : 64);
     static constexpr int MINB0 = 65536 / (TH * REGS);
     static constexpr int MINB  = MINB0 < 1 ? 1 : (MINB0 * TH > 2048 ? 2048 / TH : MINB0);
     static constexpr size_t SMEM = size_t(EPB) * NCUBE * CUBE * sizeof(T);
