@@ -32,7 +32,9 @@
 // (A_0 + A_1) B_01, i.e. its lines are added to (0, 1), (1, 0) and to one more
 // line of p = 1 whose table row is B_01 (kept in the unused slot (1, nm-1)).
 //
-// Measured on a B200 (us per call, FP64, before -> with line kernels): prism
+// Measured on a B200 (us per call, FP64, before -> with the first line kernels; a
+// shared-memory layout without conflicts, shared index work and the geometry's
+// prefetch came later): prism
 // BwdTrans 5 modes x 13718 elements 70.6 -> 21.2; hexahedral IProduct 4 modes at 8
 // points x 10648 82 -> 23.6; straight-sided tet IProductWRTDerivBase 5 modes x
 // 24576 145.9 -> 55.6; hexahedral PhysDeriv 8 points x 13824 189 -> 163; curved tet
@@ -79,6 +81,9 @@ template <typename T> struct LineArgs
     const double *geoc; // [e][kGeoc] (straight-sided), else NULL
     const T *tB1;  // Tet Modified_B table [(p,q)][j]
     const T *tB2;  // Prism Modified_B [(p,r)][k], Tet Modified_C [(p,q,r)][k]
+    const T *tC;   // the table row of every coefficient, [k][coefficient]
+    const unsigned *pairs; // Tet (p, q): p | q << 4 | modes << 8 | first << 12
+    const unsigned *coefs; // of every coefficient: p | q << 4 | fold << 8
     const int *gmap;
     const double *gsign;
     const int *skip;
@@ -86,61 +91,138 @@ template <typename T> struct LineArgs
     T lambda;
     int nelmt, nm;
     int epb; // elements per CTA of this launch
+    const uint2 *lanes; // each thread's lines along directions 1 and 2 (DEALT kernels):
+                        // offset | x << 16 | y << 20 | element << 24
 };
 
 // ---- shared-memory layout ------------------------------------------------
-// A cube's entry (a, b, c) sits at a*PS + b*RS + c. Lines along a are read by
-// lanes (b, c), along b by lanes (a, c), along c by lanes (a, b), each pair
-// with its second index fastest; the strides are those with the fewest bank
-// wavefronts over the three. A row of 4 or 8 entries is also rotated by the
-// exclusive-or of c with b, which makes all three conflict free.
-constexpr int LineWavefronts(int n1, int n2, int s1, int s2, int banks)
-{
-    int total = 0;
-    for (int g = 0; g < 3; ++g) // three groups of `banks` lanes
-    {
-        int hits[32] = {};
-        int worst    = 0;
-        for (int l = 0; l < banks; ++l)
-        {
-            const int lane = g * banks + l;
-            if (lane >= n1 * n2)
-                break;
-            const int b = ((lane / n2) * s1 + (lane % n2) * s2) % banks;
-            if (++hits[b] > worst)
-                worst = hits[b];
-        }
-        total += worst;
-    }
-    return total;
-}
-
+// A cube's entry (a, b, c) sits at a*ps + b*k2 + c, elements `cube` apart. Lines
+// along a are walked by lanes (b, c) in the arrays' order. Which lane walks which
+// line along b (a line per (a, c)) or c (per (a, b)) is free: a table
+// (LineLanes) deals them out so that the lanes of one shared-memory phase (16
+// in FP64, 32 in FP32) start in different banks. The strides are those for which
+// the lines spread most evenly over the banks. A row of 4 or 8 entries may
+// instead be rotated by the exclusive-or of c with b, with lanes in line order,
+// where that needs fewer wavefronts (e.g. 8 points: none in conflict).
 struct LineLayout
 {
-    int rs, ps;
+    int ps, cube;
+    bool rotate;
 };
 
-constexpr LineLayout LineStrides(int k0, int k1, int k2, int banks)
+// wavefronts of one access by all of a CTA's lanes, lines (x, y) in order:
+// entry 0 at e*cube + x*sx + y*sy, entry p of a rotated layout at the address
+// that `kind` (0, 1, 2: lines along a, b, c) gives
+constexpr int LineOrdered(int kind, int k0, int k1, int k2, int epb, int banks, LineLayout l)
 {
-    LineLayout best = {k2, k1 * k2 + k2};
-    if (k2 == 4 || k2 == 8)
-        return best;
-    int cost = 1 << 30;
-    for (int rs = k2; rs <= k2 + 1; ++rs)
-        for (int ps = k1 * rs; ps < k1 * rs + 16; ++ps)
+    const int n1 = kind == 0 ? k1 : k0, n2 = kind == 2 ? k1 : k2;
+    const int len = kind == 0 ? k0 : (kind == 1 ? k1 : k2);
+    const int pos = l.rotate ? len : 1; // otherwise every entry as the first
+    int total     = 0;
+    for (int p = 0; p < pos; ++p)
+        for (int t0 = 0; t0 < epb * n1 * n2; t0 += banks)
         {
-            // lines along the register direction are the most frequent
-            const int c = (3 * LineWavefronts(k1, k2, rs, 1, banks) +
-                           2 * LineWavefronts(k0, k2, ps, 1, banks) +
-                           2 * LineWavefronts(k0, k1, ps, rs, banks)) * 64 + ps - k1 * k2;
+            int hits[32] = {};
+            int worst    = 0;
+            for (int t = t0; t < t0 + banks && t < epb * n1 * n2; ++t)
+            {
+                const int e = t / (n1 * n2), x = t / n2 % n1, y = t % n2;
+                const int a = kind == 0 ? p : x, b = kind == 0 ? x : (kind == 1 ? p : y);
+                const int c = kind == 2 ? p : y;
+                const int at =
+                    e * l.cube + a * l.ps + b * k2 + (l.rotate ? (c ^ (b & (k2 - 1))) : c);
+                if (++hits[at % banks] > worst)
+                    worst = hits[at % banks];
+            }
+            total += worst;
+        }
+    return (total + pos - 1) / pos;
+}
+
+struct LineCounts
+{
+    int n[32];
+};
+
+// lines of one element per starting bank
+constexpr LineCounts LineBanks(int n1, int s1, int n2, int s2, int banks)
+{
+    LineCounts h = {};
+    for (int x = 0; x < n1; ++x)
+        for (int y = 0; y < n2; ++y)
+            ++h.n[(x * s1 + y * s2) % banks];
+    return h;
+}
+
+// wavefronts when the CTA's lines are dealt out by bank over `th` lanes
+constexpr int LineDealt(const LineCounts &h, int shift, int epb, int banks, int th)
+{
+    const int phases = th / banks;
+    int most = 0, over = 0;
+    for (int b = 0; b < banks; ++b)
+    {
+        int n = 0;
+        for (int e = 0; e < epb; ++e)
+            n += h.n[(b + (banks - shift) * e) % banks];
+        most = n > most ? n : most;
+        over += n > phases ? n - phases : 0;
+    }
+    return (most < phases ? most : phases) + over;
+}
+
+// about the accesses of the Helmholtz operator per line and direction
+constexpr int LineCost(int r, int b, int c, int k0, int k1, int k2)
+{
+    return 8 * k0 * r + 7 * k1 * b + 6 * k2 * c;
+}
+
+constexpr LineLayout LineFind(int k0, int k1, int k2, int epb, int th, int banks, int least,
+                              bool deal)
+{
+    LineLayout best = {};
+    int cost        = 1 << 30;
+    if (k2 == 4 || k2 == 8)
+    {
+        const int ps = k1 * k2 + k2;
+        best         = {ps, ((k0 * ps > least ? k0 * ps : least) + 7) & ~7, true};
+        cost         = LineCost(LineOrdered(0, k0, k1, k2, epb, banks, best),
+                                LineOrdered(1, k0, k1, k2, epb, banks, best),
+                                LineOrdered(2, k0, k1, k2, epb, banks, best), k0, k1, k2);
+    }
+    int r[32] = {};
+    for (int shift = 0; shift < banks; ++shift)
+        r[shift] = LineOrdered(0, k0, k1, k2, epb, banks, {0, shift, false});
+    for (int pad = 0; pad < 16; ++pad)
+    {
+        const int ps  = k1 * k2 + pad;
+        const auto hb = LineBanks(k0, ps, k2, 1, banks), hc = LineBanks(k0, ps, k1, k2, banks);
+        const int min = k0 * ps > least ? k0 * ps : least;
+        for (int add = 0; add < (epb > 1 ? (deal ? banks : 8) : 1); ++add)
+        {
+            const int shift    = (min + add) % banks;
+            const LineLayout l = {ps, min + add, false};
+            const int c =
+                LineCost(r[shift],
+                         deal ? LineDealt(hb, shift, epb, banks, th)
+                              : LineOrdered(1, k0, k1, k2, epb, banks, l),
+                         deal ? LineDealt(hc, shift, epb, banks, th)
+                              : LineOrdered(2, k0, k1, k2, epb, banks, l), k0, k1, k2);
             if (c < cost)
             {
                 cost = c;
-                best = {rs, ps};
+                best = {ps, min + add, false};
             }
         }
+    }
     return best;
 }
+
+// one search per set of sizes, whatever the operator
+template <int K0, int K1, int K2, int EPB, int TH, int BANKS, int LEAST, bool DEAL>
+struct LineLayoutOf
+{
+    static constexpr LineLayout V = LineFind(K0, K1, K2, EPB, TH, BANKS, LEAST, DEAL);
+};
 
 template <int SHAPE, int NM, int NQ, int OP, typename T> struct LineDims
 {
@@ -158,13 +240,7 @@ template <int SHAPE, int NM, int NQ, int OP, typename T> struct LineDims
                               : SHAPE == NKB_PRISM ? NM * NP
                                                    : NM * (NM + 1) * (NM + 2) / 6;
     static constexpr int XR = SHAPE == NKB_HEX ? NM | 1 : 1; // coefficient row stride
-    static constexpr int BANKS = 128 / int(sizeof(T));
-    static constexpr LineLayout LAY = LineStrides(K0, K1, K2, BANKS);
-    static constexpr int RS = LAY.rs, PS = LAY.ps;
-    static constexpr bool XOR = K2 == 4 || K2 == 8;
-    static constexpr int CUBE0 = K0 * PS;
     static constexpr int XSIZE = SHAPE == NKB_HEX ? NM * NM * XR : NC;
-    static constexpr int CUBE  = ((CUBE0 > XSIZE ? CUBE0 : XSIZE) + 7) & ~7;
     static constexpr int NCUBE = OP == LN_IP ? 1 : (OP == LN_BWD ? 2 : 3);
     // threads: one per line of the direction with the most lines
     static constexpr int LA = K1 * K2, LB = K0 * K2, LC = K0 * K1;
@@ -193,19 +269,30 @@ template <int SHAPE, int NM, int NQ, int OP, typename T> struct LineDims
     }
     static constexpr int EPB = Epb();
     static constexpr int TH  = (EPB * LMAX + 31) / 32 * 32;
+    static constexpr int BANKS = 128 / int(sizeof(T));
+    // without derivatives only lines of modes are walked in directions 1 and 2:
+    // lanes stay in order, so that whole warps are left idle
+    static constexpr bool DEAL = OP != LN_BWD && OP != LN_IP;
+    static constexpr LineLayout LAY = LineLayoutOf<K0, K1, K2, EPB, TH, BANKS, XSIZE, DEAL>::V;
+    static constexpr int PS = LAY.ps, CUBE = LAY.cube;
+    static constexpr bool DEALT = DEAL && !LAY.rotate && EPB < 31;
+    static_assert(EPB * CUBE < 65536, "line offsets have 16 bits");
     // register budget per thread: the lowest that spills (next to) nothing. Warps
     // in flight hide the barriers and the shared-memory latency: at 80 instead of
     // 128 registers the FP64 Helmholtz operator took 87 instead of 118 us (hex, 8
     // modes x 7140), 103 instead of 143 (9 x 5172), 115 instead of 184 (tet, 8 x
     // 10241); FP32 at 48 instead of 64 gained 0-25 %
-        static constexpr int REGS = sizeof(T) == 8 ? (K0 <= 10 ? 80 : 96) : (K0 <= 9 ? 48 : 64);
+        // (PhysDeriv's FP64 chain rule and LinearADR's extra rows take more)
+    static constexpr int REGS =
+        sizeof(T) == 8 ? (K0 <= (OP == LN_ADR ? 9 : 10) ? 80 : 96)
+                       : (OP == LN_PD && SHAPE == NKB_TET ? 56 : (K0 <= 9 ? 48 : 64));
     static constexpr int MINB0 = 65536 / (TH * REGS);
     static constexpr int MINB  = MINB0 < 1 ? 1 : (MINB0 * TH > 2048 ? 2048 / TH : MINB0);
     static constexpr size_t SMEM = size_t(EPB) * NCUBE * CUBE * sizeof(T);
 
     __device__ static __forceinline__ int Idx(int a, int b, int c)
     {
-        return a * PS + b * RS + (XOR ? (c ^ (b & (K2 - 1))) : c);
+        return a * PS + b * K2 + (LAY.rotate ? (c ^ (b & (K2 - 1))) : c);
     }
     // position in the mesh's point order (first direction fastest)
     __device__ static __forceinline__ int Natural(int a, int b, int c)
@@ -303,25 +390,10 @@ __device__ __forceinline__ void LineMulT(const T *__restrict__ tab, const T (&in
         }
 }
 
-// (p, q) of a Tet pair index (nm <= NM modes)
-template <int NM> __device__ __forceinline__ void TetPairOf(int nm, int pair, int &p, int &q)
+struct LineOf
 {
-    p = 0;
-    q = pair;
-#pragma unroll
-    for (int pp = 0; pp < NM - 1; ++pp)
-        if (q >= nm - p)
-        {
-            q -= nm - p;
-            ++p;
-        }
-}
-// first coefficient of the Tet (p, q, 0) column
-__device__ __forceinline__ int TetColumn(int nm, int p, int q)
-{
-    const int n = nm - p; // sum over p' < p of T(nm - p'), T(n) = n (n+1) / 2
-    return nm * (nm + 1) * (nm + 2) / 6 - n * (n + 1) * (n + 2) / 6 + q * n - q * (q - 1) / 2;
-}
+    int e, at, x, y; // element of the CTA, offset of the line, its two indices
+};
 
 template <int SHAPE, int NM, int NQ, int OP, typename T>
 __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
@@ -348,7 +420,7 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
     const bool curved = a.geoc == nullptr;
     const int nm      = VAR ? a.nm : NM, nm2 = nm * nm, np = nm * (nm + 1) / 2;
     const int nc      = HEX ? nm2 * nm : (TET ? nm * (nm + 1) * (nm + 2) / 6 : nm * np);
-    if ((HELM || OP == LN_IPD) && tid == 0 && curved)
+    if ((HELM || OP == LN_IPD ) && tid == 0 && curved)
         BulkPrefetchL2(a.geo + e0 * a.gstride, uint32_t(ne * a.gstride * long(sizeof(T))));
 
     // this thread's line along the register direction
@@ -357,6 +429,61 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
     const bool ract = re < ne;
     const int rbase = re * CUBE + L::Idx(0, rj, rk);
     const long rgeo = (e0 + re) * a.gstride + rl;
+
+    // its lines along directions 1 (a, c) and 2 (a, b)
+    uint2 lanes;
+    if constexpr (L::DEALT)
+        lanes = __ldg(a.lanes + tid);
+    // the thread's line along `dir` if its x < n1 and y < n2
+    auto line = [&](int dir, int n1, int n2) -> LineOf {
+        int e, at, x, y;
+        if constexpr (L::DEALT)
+        {
+            const unsigned w = dir == 1 ? lanes.x : lanes.y;
+            e = w >> 24, at = w & 0xffff, x = w >> 16 & 15, y = w >> 20 & 15;
+        }
+        else
+        {
+            const int c2 = dir == 1 ? K2 : K1;
+            e = tid / (K0 * c2), x = tid / c2 % K0, y = tid % c2;
+            at = e * CUBE + x * PS + (dir == 1 ? (L::LAY.rotate ? 0 : y) : y * K2);
+        }
+        return {x < n1 && y < n2 ? e : 31, at, x, y};
+    };
+    // entry j of a line along direction 1, k of one along direction 2
+    auto at1 = [&](const LineOf &l, int j) {
+        return l.at + j * K2 + (L::LAY.rotate ? (l.y ^ (j & (K2 - 1))) : 0);
+    };
+    auto at2 = [&](const LineOf &l, int k) {
+        return l.at + (L::LAY.rotate ? (k ^ (l.y & (K2 - 1))) : k);
+    };
+
+    // the CTA's points in the arrays' order, fn(element, point, i, j, k): a point's
+    // indices are worked out once for all elements, or, with few elements, per
+    // point so that several are in flight
+    auto each_point = [&](auto fn) {
+        if constexpr (L::EPB >= 2)
+        {
+            constexpr int U = OP == LN_IPD ? 2 : (L::EPB < 4 ? L::EPB : 4), UN = L::EPB == 2 ? 2 : 1;
+#pragma unroll(UN)
+            for (int n = tid; n < NT; n += TH)
+            {
+                const int i = n % K0, j = n / K0 % K1, k = n / (K0 * K1);
+#pragma unroll(U)
+                for (int e = 0; e < ne; ++e)
+                    fn(e, n, i, j, k);
+            }
+        }
+        else
+        {
+#pragma unroll 2
+            for (int t = tid; t < ne * NT; t += TH)
+            {
+                const int e = t / NT, n = t - e * NT;
+                fn(e, n, n % K0, n / K0 % K1, n / (K0 * K1));
+            }
+        }
+    };
 
     T u[K0], f[K0];
 
@@ -424,32 +551,20 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
             {
                 const int g = it / items, item = it - g * items;
                 const int pair = item / K2, k = item - pair * K2;
-                int p, q, xo, row, len, fold = -1;
-                T ft = 0;
+                int p, q, len, row, xo;
                 if constexpr (TET)
                 {
-                    TetPairOf<NM>(nm, pair, p, q);
-                    xo = row = TetColumn(nm, p, q);
-                    len      = nm - p - q;
-                    if (p + q == 1)
-                    {
-                        fold = 1;
-                        ft   = __ldg(a.tB2 + K2 + k);
-                    }
+                    const unsigned w = __ldg(a.pairs + pair);
+                    p = w & 15, q = w >> 4 & 15, len = w >> 8 & 15, row = xo = w >> 12;
                 }
                 else
                 {
-                    p   = pair / nm;
-                    q   = pair - p * nm;
-                    row = p * nm - p * (p - 1) / 2;
-                    len = nm - p;
-                    xo  = nm * row + q * len;
-                    if (p == 1)
-                    {
-                        fold = q * nm + 1;
-                        ft   = __ldg(a.tB2 + K2 + k);
-                    }
+                    p = pair / nm, q = pair - p * nm, len = nm - p;
+                    row = p * nm - p * (p - 1) / 2, xo = nm * row + q * len;
                 }
+                // the coefficient folded into this line
+                const int fold = TET ? (p + q == 1 ? 1 : -1) : (p == 1 ? q * nm + 1 : -1);
+                const T ft     = fold >= 0 ? __ldg(a.tB2 + K2 + k) : T(0);
                 T tab[NM];
 #pragma unroll
                 for (int r = 0; r < NM; ++r)
@@ -498,19 +613,17 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
         }
         else
         {
-            const int e = tid / (nm * K2), pk = tid - e * nm * K2;
-            const int p = pk / K2, k = pk - p * K2;
-            if (e < ne)
+            if (const LineOf l = line(1, nm, K2); l.e < ne)
             {
                 T w[NM], s[K1];
 #pragma unroll
                 for (int q = 0; q < NM; ++q)
                     if (!VAR || q < nm)
-                        w[q] = A[e * CUBE + L::Idx(p, q, k)];
+                        w[q] = A[at1(l, q)];
                 LineMul<VAR>(c.B1, w, s, nm);
 #pragma unroll
                 for (int j = 0; j < K1; ++j)
-                    Bc[e * CUBE + L::Idx(p, j, k)] = s[j];
+                    Bc[at1(l, j)] = s[j];
             }
         }
         __syncthreads();
@@ -543,12 +656,9 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
             {
                 __syncthreads();
                 T *o = a.out0 + e0 * NT;
-                for (int t = tid; t < ne * NT; t += TH)
-                {
-                    const int e = t / NT, n = t - e * NT;
-                    const int i = n % K0, j = n / K0 % K1, k = n / (K0 * K1);
-                    o[t] = S0[e * CUBE + L::Idx(i, j, k)];
-                }
+                each_point([&](int e, int n, int i, int j, int k) {
+                    o[e * NT + n] = S0[e * CUBE + L::Idx(i, j, k)];
+                });
             }
             return;
         }
@@ -623,11 +733,7 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
         }
         else
         {
-#pragma unroll 2
-            for (int t = tid; t < ne * NT; t += TH)
-            {
-                const int e = t / NT, n = t - e * NT;
-                const int i = n % K0, j = n / K0 % K1, k = n / (K0 * K1);
+            each_point([&](int e, int n, int i, int j, int k) {
                 T v0, v1, v2;
                 point(e0 + e, n, i, j, k, v0, v1, v2);
                 const int s = e * CUBE + L::Idx(i, j, k);
@@ -637,7 +743,7 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
                     S1[s] = v1;
                     S2[s] = v2;
                 }
-            }
+            });
             __syncthreads();
             if (ract)
             {
@@ -655,13 +761,6 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
         }
     }
 
-    // lines along directions 1 and 2, one of each per thread
-    const int be = tid / L::LB, bl = tid - be * L::LB;
-    const int bi = bl / K2, bk = bl - bi * K2;
-    const int ce = tid / L::LC, cl = tid - ce * L::LC;
-    const int ci = cl / K1, cj = cl - ci * K1;
-    const int bbase = be * CUBE + bi * PS, cbase = ce * CUBE + ci * PS;
-
     if constexpr (HELM || OP == LN_PD)
     {
         // ---------------- gradient -----------------------------------------
@@ -669,27 +768,27 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
         if (ract)
             LineMul(c.D0, u, g0);
         __syncthreads();
-        if (be < ne)
+        if (const LineOf l = line(1, K0, K2); l.e < ne)
         {
             T v[K1], g[K1];
 #pragma unroll
             for (int j = 0; j < K1; ++j)
-                v[j] = S0[bbase + L::Idx(0, j, bk)];
+                v[j] = S0[at1(l, j)];
             LineMul(c.D1, v, g);
 #pragma unroll
             for (int j = 0; j < K1; ++j)
-                S1[bbase + L::Idx(0, j, bk)] = g[j];
+                S1[at1(l, j)] = g[j];
         }
-        if (ce < ne)
+        if (const LineOf l = line(2, K0, K1); l.e < ne)
         {
             T v[K2], g[K2];
 #pragma unroll
             for (int k = 0; k < K2; ++k)
-                v[k] = S0[cbase + L::Idx(0, cj, k)];
+                v[k] = S0[at2(l, k)];
             LineMul(c.D2, v, g);
 #pragma unroll
             for (int k = 0; k < K2; ++k)
-                S2[cbase + L::Idx(0, cj, k)] = g[k];
+                S2[at2(l, k)] = g[k];
         }
         __syncthreads();
         if constexpr (OP == LN_PD)
@@ -803,34 +902,34 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
     if constexpr (HELM || OP == LN_IPD)
     {
         // ---------------- transposed gradient, in place ----------------------
-        if (be < ne)
+        if (const LineOf l = line(1, K0, K2); l.e < ne)
         {
             T v[K1], g[K1];
 #pragma unroll
             for (int j = 0; j < K1; ++j)
-                v[j] = S1[bbase + L::Idx(0, j, bk)];
+                v[j] = S1[at1(l, j)];
             LineMulT(c.D1, v, g);
 #pragma unroll
             for (int j = 0; j < K1; ++j)
-                S1[bbase + L::Idx(0, j, bk)] = g[j];
+                S1[at1(l, j)] = g[j];
         }
-        if (ce < ne)
+        if (const LineOf l = line(2, K0, K1); l.e < ne)
         {
             T v[K2], g[K2];
 #pragma unroll
             for (int k = 0; k < K2; ++k)
-                v[k] = S2[cbase + L::Idx(0, cj, k)];
+                v[k] = S2[at2(l, k)];
             LineMulT(c.D2, v, g);
 #pragma unroll
             for (int k = 0; k < K2; ++k)
-                S2[cbase + L::Idx(0, cj, k)] = g[k];
+                S2[at2(l, k)] = g[k];
         }
         __syncthreads();
         if (ract)
         {
 #pragma unroll
             for (int i = 0; i < K0; ++i)
-                f[i] += S1[rbase + i * PS] + S2[rbase + i * PS];
+                f[i] = (f[i] + S2[rbase + i * PS]) + S1[rbase + i * PS];
         }
     }
 
@@ -846,47 +945,41 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
                 S0[rbase + i * PS] = f[i];
         }
         __syncthreads();
-        if (ce < ne)
+        if (const LineOf l = line(2, K0, K1); l.e < ne)
         {
             T v[K2], s[NM];
 #pragma unroll
             for (int k = 0; k < K2; ++k)
-                v[k] = S0[cbase + L::Idx(0, cj, k)];
+                v[k] = S0[at2(l, k)];
             LineMulT<VAR>(c.B2, v, s, nm);
 #pragma unroll
             for (int r = 0; r < NM; ++r)
                 if (!VAR || r < nm)
-                    S0[cbase + L::Idx(0, cj, r)] = s[r];
+                    S0[at2(l, r)] = s[r];
+        }
+        __syncthreads();
+        if (const LineOf l = line(1, K0, nm); l.e < ne)
+        {
+            T v[K1], s[NM];
+#pragma unroll
+            for (int j = 0; j < K1; ++j)
+                v[j] = S0[at1(l, j)];
+            LineMulT<VAR>(c.B1, v, s, nm);
+#pragma unroll
+            for (int q = 0; q < NM; ++q)
+                if (!VAR || q < nm)
+                    S0[at1(l, q)] = s[q];
         }
         __syncthreads();
         {
-            const int e = tid / (K0 * nm), ir = tid - e * K0 * nm;
-            const int i = ir / nm, r = ir - i * nm;
-            if (e < ne)
-            {
-                T v[K1], s[NM];
-#pragma unroll
-                for (int j = 0; j < K1; ++j)
-                    v[j] = S0[e * CUBE + L::Idx(i, j, r)];
-                LineMulT<VAR>(c.B1, v, s, nm);
-#pragma unroll
-                for (int q = 0; q < NM; ++q)
-                    if (!VAR || q < nm)
-                        S0[e * CUBE + L::Idx(i, q, r)] = s[q];
-            }
-        }
-        __syncthreads();
-        {
-            const int e = tid / nm2, qr = tid - e * nm2;
-            const int q = qr / nm, r = qr - q * nm;
-            if (e < ne)
+            if (ract && rj < nm && rk < nm)
             {
                 T v[K0], s[NM];
 #pragma unroll
                 for (int i = 0; i < K0; ++i)
-                    v[i] = S0[e * CUBE + L::Idx(i, q, r)];
+                    v[i] = S0[rbase + i * PS];
                 LineMulT<VAR>(c.B0, v, s, nm);
-                T *y = a.out0 + (e0 + e) * nc + qr;
+                T *y = a.out0 + (e0 + re) * nc + rj * nm + rk;
 #pragma unroll
                 for (int p = 0; p < NM; ++p)
                     if (!VAR || p < nm)
@@ -932,19 +1025,17 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
         }
         else
         {
-            const int e = tid / (nm * K2), pk = tid - e * nm * K2;
-            const int p = pk / K2, k = pk - p * K2;
-            if (e < ne)
+            if (const LineOf l = line(1, nm, K2); l.e < ne)
             {
                 T v[K1], s[NM];
 #pragma unroll
                 for (int j = 0; j < K1; ++j)
-                    v[j] = S0[e * CUBE + L::Idx(p, j, k)];
+                    v[j] = S0[at1(l, j)];
                 LineMulT<VAR>(c.B1, v, s, nm);
 #pragma unroll
                 for (int q = 0; q < NM; ++q)
                     if (!VAR || q < nm)
-                        S0[e * CUBE + L::Idx(p, q, k)] = s[q];
+                        S0[at1(l, q)] = s[q];
             }
         }
         __syncthreads();
@@ -954,45 +1045,12 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
         for (int it = tid; it < nc * G; it += TH)
         {
             const int g = it / nc, m = it - g * nc;
-            int p = 0, q = 0, row, rem = m;
-            bool fold; // the singular-edge / collapsed-vertex terms
-            if constexpr (TET)
-            {
-#pragma unroll
-                for (int pp = 0; pp < NM - 1; ++pp)
-                    if (rem >= (nm - p) * (nm - p + 1) / 2)
-                    {
-                        rem -= (nm - p) * (nm - p + 1) / 2;
-                        ++p;
-                    }
-#pragma unroll
-                for (int qq = 0; qq < NM - 1; ++qq)
-                    if (rem >= nm - p - q)
-                    {
-                        rem -= nm - p - q;
-                        ++q;
-                    }
-                row  = m;
-                fold = m == 1 || (p == 0 && q == 1);
-            }
-            else
-            {
-#pragma unroll
-                for (int pp = 0; pp < NM - 1; ++pp)
-                    if (rem >= nm * (nm - p))
-                    {
-                        rem -= nm * (nm - p);
-                        ++p;
-                    }
-                q           = rem / (nm - p);
-                const int r = rem - q * (nm - p);
-                row         = p * nm - p * (p - 1) / 2 + r;
-                fold        = p == 0 && r == 1;
-            }
+            const unsigned w = __ldg(a.coefs + m);
+            const int p = w & 15, q = (w >> 4) & 15, fold = w >> 8;
             T tab[K2];
 #pragma unroll
             for (int k = 0; k < K2; ++k)
-                tab[k] = __ldg(a.tB2 + row * K2 + k);
+                tab[k] = __ldg(a.tC + k * nc + m);
             for (int e = g; e < ne; e += G)
             {
                 const T *s = S0 + e * CUBE;
@@ -1007,7 +1065,7 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
                     {
                         if (!TET)
                             v[k] += s[L::Idx(1, q, k)];
-                        else if (m == 1)
+                        else if (fold == 2)
                             v[k] += (s[L::Idx(0, 1, k)] + s[L::Idx(1, nm - 1, k)]) +
                                     s[L::Idx(1, 0, k)];
                         else
@@ -1074,6 +1132,101 @@ void LineBuildTabs(const nkb_op *op, std::vector<unsigned char> &blob)
     std::memcpy(blob.data(), &t, sizeof(t));
 }
 
+// deals the lines (x, y) of epb elements out to th lanes, at most one per bank to
+// the lanes of a phase where the banks allow it (words of LineArgs::lanes)
+inline void LineDeal(int epb, int cube, int n1, int s1, int n2, int s2, int banks, int th,
+                     bool in_order, std::vector<unsigned> &lanes)
+{
+    lanes.assign(th, 31u << 24); // element 31: none
+    std::vector<std::vector<unsigned>> by_bank(banks);
+    for (int e = 0, t = 0; e < epb; ++e)
+        for (int x = 0; x < n1; ++x)
+            for (int y = 0; y < n2; ++y, ++t)
+            {
+                const int at     = e * cube + x * s1 + y * s2;
+                const unsigned w = unsigned(at | x << 16 | y << 20) | unsigned(e) << 24;
+                if (in_order)
+                    lanes[t] = w;
+                else
+                    by_bank[at % banks].push_back(w);
+            }
+    std::vector<int> spare;
+    for (int t0 = 0; t0 < th && !in_order; t0 += banks)
+        for (int b = 0; b < banks; ++b)
+        {
+            if (by_bank[b].empty())
+            {
+                spare.push_back(t0 + b);
+                continue;
+            }
+            lanes[t0 + b] = by_bank[b].back();
+            by_bank[b].pop_back();
+        }
+    for (auto &rest : by_bank)
+        for (unsigned line : rest)
+        {
+            lanes[spare.back()] = line;
+            spare.pop_back();
+        }
+}
+
+// device tables of an operator, one allocation: the table row of every
+// coefficient ([k][coefficient]), then lanes, pairs and coefs of LineArgs
+template <int SHAPE, int NM, int NQ, int OP, typename T> int LineBuildAux(nkb_op *op)
+{
+    using L      = LineDims<SHAPE, NM, NQ, OP, T>;
+    const int nm = op->nm;
+    std::vector<T> rows;
+    std::vector<unsigned> words;
+    // dealt out for full CTAs, in order for the smaller ones of small collections
+    for (int in_order = 0; in_order < 2 && L::DEALT; ++in_order)
+    {
+        std::vector<unsigned> l1, l2;
+        LineDeal(L::EPB, L::CUBE, L::K0, L::PS, L::K2, 1, L::BANKS, L::TH, in_order, l1);
+        LineDeal(L::EPB, L::CUBE, L::K0, L::PS, L::K1, L::K2, L::BANKS, L::TH, in_order, l2);
+        for (int t = 0; t < L::TH; ++t)
+        {
+            words.push_back(l1[t]);
+            words.push_back(l2[t]);
+        }
+    }
+    if (SHAPE != NKB_HEX && OP != LN_PD)
+    {
+        std::vector<unsigned> coefs;
+        std::vector<int> row;
+        for (int p = 0, first = 0; p < nm; ++p)
+            for (int q = 0; q < (SHAPE == NKB_TET ? nm - p : nm); ++q)
+            {
+                const int len = SHAPE == NKB_TET ? nm - p - q : nm - p;
+                if (SHAPE == NKB_TET)
+                    words.push_back(unsigned(p | q << 4 | len << 8 | first << 12));
+                for (int r = 0; r < len; ++r, ++first)
+                {
+                    // prism (0, q, 1) and tet (0, 1, r): one more line; tet (0, 0, 1): three
+                    const int fold = SHAPE == NKB_TET ? (first == 1 ? 2 : p == 0 && q == 1)
+                                                      : p == 0 && r == 1;
+                    coefs.push_back(unsigned(p | q << 4 | fold << 8));
+                    row.push_back(SHAPE == NKB_TET ? first : p * nm - p * (p - 1) / 2 + r);
+                }
+            }
+        words.insert(words.end(), coefs.begin(), coefs.end());
+        for (int k = 0; k < L::K2; ++k)
+            for (int m : row)
+                rows.push_back(T(op->hB[2][size_t(m) * L::K2 + k]));
+    }
+    if (rows.size() % 2)
+        rows.push_back(T(0));
+    const size_t nr = rows.size() * sizeof(T), nw = words.size() * sizeof(unsigned);
+    std::vector<unsigned char> image(nr + nw);
+    if (nr)
+        std::memcpy(image.data(), rows.data(), nr);
+    std::memcpy(image.data() + nr, words.data(), nw);
+    op->line_words = nr;
+    NKB_CUDA_TRY(cudaMalloc(&op->line_aux, image.size()));
+    NKB_CUDA_TRY(cudaMemcpy(op->line_aux, image.data(), image.size(), cudaMemcpyHostToDevice));
+    return NKB_OK;
+}
+
 // one kernel: build its tables (setup) or launch it
 template <int SHAPE, int NM, int NQ, int OP, typename T>
 int LineOne(nkb_op *setup, const nkb_op *op, const LineArgs<T> *a, cudaStream_t s)
@@ -1084,6 +1237,9 @@ int LineOne(nkb_op *setup, const nkb_op *op, const LineArgs<T> *a, cudaStream_t 
     if (setup)
     {
         LineBuildTabs<SHAPE, NM, NQ, OP, T>(setup, setup->line_tabs);
+        const int rc = LineBuildAux<SHAPE, NM, NQ, OP, T>(setup);
+        if (rc)
+            return rc;
         NKB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           int(L::SMEM)));
         return NKB_OK;
@@ -1095,6 +1251,12 @@ int LineOne(nkb_op *setup, const nkb_op *op, const LineArgs<T> *a, cudaStream_t 
     run.epb           = std::min(L::EPB, (op->nelmt + slots - 1) / slots);
     const unsigned nb = unsigned((op->nelmt + run.epb - 1) / run.epb);
     const unsigned th = unsigned((run.epb * L::LMAX + 31) / 32 * 32);
+    const unsigned char *aux = static_cast<const unsigned char *>(op->line_aux);
+    const unsigned *words    = reinterpret_cast<const unsigned *>(aux + op->line_words);
+    run.tC    = reinterpret_cast<const T *>(aux);
+    run.lanes = reinterpret_cast<const uint2 *>(words) + (run.epb == L::EPB ? 0 : L::TH);
+    run.pairs = words + (L::DEALT ? 4 * L::TH : 0);
+    run.coefs = run.pairs + (SHAPE == NKB_TET ? op->nm * (op->nm + 1) / 2 : 0);
     void *params[2]   = {&run, const_cast<unsigned char *>(op->line_tabs.data())};
     NKB_CUDA_TRY(cudaLaunchKernel((const void *)kern, dim3(nb), dim3(th), params,
                                   size_t(run.epb) * L::NCUBE * L::CUBE * sizeof(T), s));

@@ -37,10 +37,12 @@ struct nkb_op
 
     // line kernels (nkb_line.cu): their tables in parameter layout (empty: not
     // used); packed geometry with the third direction fastest; 16 values per
-    // straight-sided element
+    // straight-sided element; tables and index words on the device
     std::vector<unsigned char> line_tabs;
     int geo_perm = 0;
     double *geoc = nullptr;
+    void *line_aux    = nullptr;
+    size_t line_words = 0; // offset of its words
 
     // kernel selection (nkb_hex.cu): 0 generic, >0 tuned variant
     int variant     = 0;

@@ -1279,6 +1279,7 @@ extern "C" void nkb_op_destroy(nkb_op *op)
     cudaFree(op->geo);
     cudaFree(op->geo32);
     cudaFree(op->geoc);
+    cudaFree(op->line_aux);
     cudaFree(op->scratch);
     cudaFree(op->d_err);
     cudaFree(op->tc_tab);
