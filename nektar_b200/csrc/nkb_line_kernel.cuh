@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
     const bool curved = a.geoc == nullptr;
     const int nm      = VAR ? a.nm : NM, nm2 = nm * nm, np = nm * (nm + 1) / 2;
     const int nc      = HEX ? nm2 * nm : (TET ? nm * (nm + 1) * (nm + 2) / 6 : nm * np);
-    if ((HELM || OP == LN_IPD ) && tid == 0 && curved)
+    if ((HELM || OP == LN_IPD || OP == LN_PD) && tid == 0 && curved)
         BulkPrefetchL2(a.geo + e0 * a.gstride, uint32_t(ne * a.gstride * long(sizeof(T))));
 
     // this thread's line along the register direction
