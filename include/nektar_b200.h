@@ -284,7 +284,7 @@ int nkb_op_check_error(nkb_op *op);
  * make the wait run out; no reference counterpart. */
 int nkb_op_set_wait_limit(nkb_op *op, int polls);
 
-/* Name of the device kernel the operator runs (the autotuned choice; gather =
+/* Name of the device kernel the operator runs (chosen at creation; gather =
  * 1: the one used when a system gathers its input through the map). For
  * reports; no reference counterpart. */
 const char *nkb_op_kernel(const nkb_op *op, int gather);

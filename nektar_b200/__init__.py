@@ -253,7 +253,7 @@ class Operator:
             check(fn(self.h, x_ptr, out0, out1, out2, stream))
 
     def kernel(self, gather=False):
-        """Name of the device kernel the operator runs (autotuned choice)."""
+        """Name of the device kernel the operator runs (chosen at creation)."""
         return lib().nkb_op_kernel(self.h, int(bool(gather))).decode()
 
     def last_kernel_ms(self):

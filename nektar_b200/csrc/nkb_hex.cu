@@ -1,23 +1,9 @@
-// Tuned Hex Helmholtz kernel and kernel selection for the element operators.
-//
-// The Hex Helmholtz operator (the reference's fusedKernel3D,
-// MatrixFreeOps/Helmholtz.h:549-599, in the collocation form described in
-// nkb_ops.cu) for nq = nm + 1 points per direction, nm = 2..11, FP64 or FP32.
-//
-// Work decomposition: one thread per (i, j) column of the nq x nq slab of an
-// element; the third direction k lives in registers. So the contraction over
-// r in BwdTrans, d/dxi_2, its transpose and the first inner-product stage are
-// register-only; the i- and j-direction contractions read shared memory with
-// broadcast-friendly patterns (the k-plane of a column is shared by the
-// threads of a row). EPB elements share a CTA.
-//
-// Data movement: the element's packed geometry (W and the six metric terms,
-// 7 nq^3 values) is fetched by ONE bulk TMA copy per CTA issued before any
-// arithmetic, completing on an mbarrier; it streams in while BwdTrans and the
-// gradient run, and only the metric stage waits for it (bounded wait). The
-// 1-D tables are staged in shared memory (D padded to nq+1 columns).
-// Coefficients are read coalesced, either contiguous (Collections layout) or
-// gathered through the local-to-global map (the CG matvec).
+// Kernel selection for the element operators, and the Hex Helmholtz kernels that
+// NKB_HEX_VARIANT requests instead of the line kernels (nkb_line_kernel.cuh):
+// k_hex_helm, one thread per (i, j) column of the nq x nq slab with the third
+// direction in registers and the packed geometry fetched by one bulk TMA copy per
+// CTA that completes on an mbarrier (bounded wait), and the tcgen05 kernel of
+// nkb_hex_tc.cuh. The line kernels were faster at every order in FP64 and FP32.
 #include "nkb_hex_kernel.cuh"
 #include "nkb_op.h"
 
@@ -53,22 +39,6 @@ int SmCount(int device)
     return counts[device];
 }
 
-int ResidentCtas(const void *fn, int threads, size_t smem)
-{
-    cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess)
-        return 1;
-    const int warps    = (threads + 31) / 32;
-    const int regs     = ((fa.numRegs + 7) / 8) * 8;                // allocation granularity
-    const long by_regs = 65536L / (long(warps) * 32 * (regs > 0 ? regs : 1));
-    const long by_smem = long(227 * 1024) / long(smem + fa.sharedSizeBytes + 1024);
-    const long by_thr  = 2048L / (long(warps) * 32);
-    long n             = by_regs < by_smem ? by_regs : by_smem;
-    n                  = n < by_thr ? n : by_thr;
-    n                  = n < 32 ? n : 32;
-    return n < 1 ? 1 : int(n);
-}
-
 static bool ForceGeneric()
 {
     const char *v = std::getenv("NKB_KERNEL");
@@ -100,8 +70,8 @@ static float Tf32HiHost(float x)
 int BuildTcTables(nkb_op *op)
 {
     const int nm = op->nm, nq = op->nq[0];
-    if (op->shape != NKB_HEX || op->optype != NKB_HELMHOLTZ || op->precision != NKB_FP32 ||
-        nm < kTcMinNm || nm > kTcMaxNm || nq != nm + 1 || op->nq[1] != nq || op->nq[2] != nq)
+    int v = 0;
+    if (!HexVariantRequested(op, &v) || v != 5)
         return NKB_OK;
     auto pad8 = [](int v) { return (v + 7) / 8 * 8; };
     const int KM = pad8(nm), KQ = pad8(nq), NQP = pad8(nq), NMN = pad8(nm);
@@ -195,89 +165,7 @@ template <typename T> static HexArgs<T> MakeHexArgs(const nkb_op *op)
     return a;
 }
 
-// Timing autotuner over the Hex variants, in the spirit of the reference's
-// CollectionOptimisation::SetWithTimings (CollectionOptimisation.cpp:393-580):
-// time each candidate on this operator's own data and keep the fastest; the
-// choice is cached per (precision, nm, element count).
 static std::mutex g_tune_mu;
-static std::map<std::tuple<int, int, int, int>, int> g_tune_cache;
-
-// The tuners time short bursts of launches. Over a whole solve the 1 kW power
-// cap lowers the SM clock more under the CUDA-core FP64 kernels than under
-// the tensor-core ones (measured at 32^3, P=6: 1810 against 1895 MHz, the
-// whole solve 3 % slower with the CUDA-core kernel that won the burst by
-// 1.6 %), so a tensor-core variant (3, 4, 5) competes with its burst time
-// scaled by this factor.
-constexpr float kTensorPreference = 0.95f;
-
-static float TunedMs(int variant, float ms)
-{
-    return (variant >= 3 && variant <= 5) ? ms * kTensorPreference : ms;
-}
-
-template <typename T> static int AutotuneHex(nkb_op *op, int *best)
-{
-    if (op->nelmt == 0)
-    {
-        *best = 1; // nothing to time: the streamed variant exists at every order
-        return NKB_OK;
-    }
-    const auto key = std::make_tuple(op->optype, op->precision, op->nm, op->nelmt);
-    {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        auto it = g_tune_cache.find(key);
-        if (it != g_tune_cache.end())
-        {
-            *best = it->second;
-            return NKB_OK;
-        }
-    }
-    const size_t n = size_t(op->nelmt) * op->nc;
-    T *buf         = nullptr;
-    if (cudaMalloc(&buf, 2 * n * sizeof(T)) != cudaSuccess)
-        return SetError(NKB_ERR_NOMEM, "autotune buffers");
-    cudaMemsetAsync(buf, 0, 2 * n * sizeof(T), op->stream);
-    HexArgs<T> a = MakeHexArgs<T>(op);
-    a.in         = buf;
-    a.out        = buf + n;
-    float best_ms = 1e30f;
-    int bi        = -1, rc = NKB_OK;
-    for (int v = 0; v < kNumHexVariants; ++v)
-    {
-        if (HexLaunchT<T>(op, a, false, op->stream, v, true) != NKB_OK)
-        {
-            ClearError();
-            continue;
-        }
-        if ((rc = HexLaunchT<T>(op, a, false, op->stream, v, false)))
-            break;
-        cudaEventRecord(op->ev0, op->stream);
-        for (int it = 0; it < 3 && !rc; ++it)
-            rc = HexLaunchT<T>(op, a, false, op->stream, v, false);
-        cudaEventRecord(op->ev1, op->stream);
-        if (rc || cudaEventSynchronize(op->ev1) != cudaSuccess)
-            break;
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, op->ev0, op->ev1);
-        if (std::getenv("NKB_TUNE_VERBOSE"))
-            std::fprintf(stderr, "hex tune nm=%d nelmt=%d fp%d variant %d: %.4f ms per launch\n",
-                         op->nm, op->nelmt, op->precision == NKB_FP64 ? 64 : 32, v, ms / 3);
-        if (TunedMs(v, ms) < best_ms)
-        {
-            best_ms = TunedMs(v, ms);
-            bi      = v;
-        }
-    }
-    cudaFree(buf);
-    if (rc)
-        return rc;
-    if (bi < 0)
-        return SetError(NKB_ERR_UNSUPPORTED, "no Hex variant could be launched");
-    *best = bi;
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune_cache[key] = bi;
-    return NKB_OK;
-}
 
 // Launch shape of the generic kernel (threads per CTA, elements per CTA),
 // timed on the operator's own sizes the same way and cached per (shape,
@@ -356,31 +244,33 @@ static bool SameTable(const std::vector<double> &a, const std::vector<double> &b
     return a.size() == b.size() && std::equal(a.begin(), a.end(), b.begin());
 }
 
+bool HexVariantRequested(const nkb_op *op, int *v)
+{
+    const char *env = std::getenv("NKB_HEX_VARIANT");
+    const int nm    = op->nm;
+    if (!env || op->shape != NKB_HEX || nm < 2 || nm > 11 || op->nq[0] != nm + 1 ||
+        (op->optype != NKB_HELMHOLTZ && op->optype != NKB_LINEAR_ADR) ||
+        !SameTable(op->hD[0], op->hD[1]) || !SameTable(op->hD[0], op->hD[2]) || ForceGeneric())
+        return false;
+    *v = std::atoi(env);
+    return *v == 0 || (*v == 5 && op->optype == NKB_HELMHOLTZ && op->precision == NKB_FP32 &&
+                       nm >= kTcMinNm && nm <= kTcMaxNm);
+}
+
 int ChooseKernel(nkb_op *op)
 {
     op->variant  = kVariantGeneric;
     if (!op->line_tabs.empty())
         return NKB_OK; // a line kernel (nkb_line.cu): nothing to choose
     const int eb = op->precision == NKB_FP64 ? 8 : 4;
-    if (op->shape == NKB_HEX && (op->optype == NKB_HELMHOLTZ || op->optype == NKB_LINEAR_ADR) &&
-        op->nm >= 2 && op->nm <= 11 &&
-        op->nq[0] == op->nm + 1 && op->nq[1] == op->nq[0] && op->nq[2] == op->nq[0] &&
-        SameTable(op->hD[0], op->hD[1]) && SameTable(op->hD[0], op->hD[2]) && !ForceGeneric())
+    int v = 0;
+    if (HexVariantRequested(op, &v))
     {
-        int v           = -1, rc;
-        const char *env = std::getenv("NKB_HEX_VARIANT");
-        if (env)
-            v = std::atoi(env);
-        if (v < 0 || v >= kNumHexVariants)
-        {
-            rc = op->precision == NKB_FP64 ? AutotuneHex<double>(op, &v) : AutotuneHex<float>(op, &v);
-            if (rc)
-                return rc;
-        }
         HexArgs<double> ad = MakeHexArgs<double>(op);
         HexArgs<float> af  = MakeHexArgs<float>(op);
-        rc = op->precision == NKB_FP64 ? HexLaunchT<double>(op, ad, false, op->stream, v, true)
-                                       : HexLaunchT<float>(op, af, false, op->stream, v, true);
+        const int rc = op->precision == NKB_FP64
+                           ? HexLaunchT<double>(op, ad, false, op->stream, v, true)
+                           : HexLaunchT<float>(op, af, false, op->stream, v, true);
         if (rc == NKB_OK)
         {
             op->variant     = kVariantHexHelm;
@@ -404,64 +294,7 @@ void FreeKernelData(nkb_op *op)
     op->kdata = nullptr;
 }
 
-template <typename T>
-static int TuneHexGatherT(nkb_op *op, const T *xin, T *yl, const int *map, const double *sign,
-                          cudaStream_t s)
-{
-    HexArgs<T> a = MakeHexArgs<T>(op);
-    a.in         = xin;
-    a.out        = yl;
-    a.gmap       = map;
-    a.gsign      = sign;
-    float best_ms = 1e30f;
-    int best = -1, rc = NKB_OK;
-    for (int v = 0; v < kNumHexVariants && !rc; ++v)
-    {
-        if (HexLaunchT<T>(op, a, true, s, v, true) != NKB_OK)
-        {
-            ClearError();
-            continue;
-        }
-        if ((rc = HexLaunchT<T>(op, a, true, s, v, false)))
-            break;
-        cudaEventRecord(op->ev0, s);
-        for (int it = 0; it < 3 && !rc; ++it)
-            rc = HexLaunchT<T>(op, a, true, s, v, false);
-        cudaEventRecord(op->ev1, s);
-        if (rc || cudaEventSynchronize(op->ev1) != cudaSuccess)
-            break;
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, op->ev0, op->ev1);
-        if (std::getenv("NKB_TUNE_VERBOSE"))
-            std::fprintf(stderr, "hex tune (gathered) nm=%d nelmt=%d fp%d variant %d: %.4f ms per "
-                                 "launch\n",
-                         op->nm, op->nelmt, op->precision == NKB_FP64 ? 64 : 32, v, ms / 3);
-        if (TunedMs(v, ms) < best_ms)
-        {
-            best_ms = TunedMs(v, ms);
-            best    = v;
-        }
-    }
-    if (rc)
-        return rc;
-    if (best >= 0)
-        op->hex_variant_gather = best;
-    return NKB_OK;
-}
-
-int TuneHexGather(nkb_op *op, const void *xin, void *yl, const int *map, const double *sign,
-                  cudaStream_t s)
-{
-    if (op->variant != kVariantHexHelm || std::getenv("NKB_HEX_VARIANT"))
-        return NKB_OK;
-    return op->precision == NKB_FP64
-               ? TuneHexGatherT<double>(op, static_cast<const double *>(xin),
-                                        static_cast<double *>(yl), map, sign, s)
-               : TuneHexGatherT<float>(op, static_cast<const float *>(xin),
-                                       static_cast<float *>(yl), map, sign, s);
-}
-
-const char *KernelName(const nkb_op *op, bool gather)
+const char *KernelName(const nkb_op *op, bool)
 {
     if (op->optype == NKB_DENSE_BLOCK)
         return "k_dense_gemv (per-element dense blocks)";
@@ -472,19 +305,9 @@ const char *KernelName(const nkb_op *op, bool gather)
             return "k_col_helm (Prism/Tet column kernel: k_line)";
         return op->line_tabs.empty() ? "k_generic" : "k_line (one thread per grid line)";
     }
-    const int v = (gather && op->hex_variant_gather >= 0) ? op->hex_variant_gather : op->hex_variant;
-    switch (v)
-    {
-        case 0: return "k_hex_helm (TMA-staged geometry)";
-        case 1: return "k_hex_helm (streamed geometry, 1 element per CTA)";
-        case 2: return "k_hex_helm (streamed geometry, 2 elements per CTA)";
-        case 3: return "k_hex_helm_mma (FP64 tensor cores)";
-        case 4: return "k_hex_helm_mma2 (FP64 tensor cores, two warps per element)";
-        case 5: return "k_hex_helm_tc (tcgen05 TF32 high/low tensor cores, FP32 accumulate)";
-        case 6: return "k_hex_helm (persistent, double-buffered TMA geometry)";
-        case 8: return "k_hex_helm (TMA-staged geometry, groups up to 72 KB)";
-        default: return "k_hex_helm (TMA-staged geometry, small groups)";
-    }
+    return op->hex_variant == 5
+               ? "k_hex_helm_tc (tcgen05 TF32 high/low tensor cores, FP32 accumulate)"
+               : "k_hex_helm (TMA-staged geometry)";
 }
 
 template <typename T>
@@ -510,8 +333,7 @@ int LaunchOp(const nkb_op *op, const T *in, T *o0, T *o1, T *o2, const int *gmap
         a.gmap       = gmap;
         a.gsign      = gsign;
         a.skip       = skip;
-        const int v = (gmap && op->hex_variant_gather >= 0) ? op->hex_variant_gather : op->hex_variant;
-        return HexLaunchT<T>(op, a, gmap != nullptr, s, v, false);
+        return HexLaunchT<T>(op, a, gmap != nullptr, s, op->hex_variant, false);
     }
     return LaunchGeneric<T>(op, in, o0, o1, o2, gmap, gsign, s, skip, lambda);
 }

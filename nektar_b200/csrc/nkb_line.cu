@@ -46,8 +46,9 @@ int LineSetup(nkb_op *op)
     const bool hex  = op->shape == NKB_HEX;
     if (EnvIs("NKB_KERNEL", "generic") || (helm && !hex && EnvIs("NKB_COL", "0")))
         return NKB_OK;
-    if (helm && hex && op->nq[0] == op->nm + 1 && std::getenv("NKB_HEX_VARIANT"))
-        return NKB_OK; // one of nkb_hex.cu's variants, by request
+    int v = 0;
+    if (HexVariantRequested(op, &v))
+        return NKB_OK; // one of nkb_hex.cu's kernels, by request
     const int rc = op->precision == NKB_FP64
                        ? LineDispatch<double>(op, op, nullptr, nullptr)
                        : LineDispatch<float>(op, op, nullptr, nullptr);

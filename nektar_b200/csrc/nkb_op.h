@@ -46,9 +46,7 @@ struct nkb_op
 
     // kernel selection (nkb_hex.cu): 0 generic, >0 tuned variant
     int variant     = 0;
-    int hex_variant = 0; // tuned Hex kernel variant chosen by the autotuner
-    int hex_variant_gather = -1; // variant for launches that gather through a
-                                 // map (timed with the system's map; -1: same)
+    int hex_variant = 0; // Hex kernel variant (NKB_HEX_VARIANT)
     int gen_epb     = 0; // generic kernel: elements per CTA (0: default)
     int gen_threads = 0; // generic kernel: threads per CTA (0: default)
     void *kdata = nullptr;
@@ -100,16 +98,13 @@ int LaunchOp(const nkb_op *op, const T *in, T *o0, T *o1, T *o2, const int *gmap
              const double *gsign, cudaStream_t s, const int *skip = nullptr,
              const double *lambda = nullptr);
 int ChooseKernel(nkb_op *op);
-// tables of the tensor-core Hex kernel (FP32 Hex Helmholtz ops, nm 2..9)
+// tables of the tensor-core Hex kernel, where it is requested
 int BuildTcTables(nkb_op *op);
 // reads and clears the operator's device error word (after its work has
 // completed): NKB_ERR_TIMEOUT when a bounded wait gave up, else NKB_OK
 int CheckOpError(nkb_op *op);
-// time the Hex variants once more with the local<-global gather a system
-// uses (xin: global vector, yl: local output) and keep the fastest for
-// gathered launches
-int TuneHexGather(nkb_op *op, const void *xin, void *yl, const int *map, const double *sign,
-                  cudaStream_t s);
+// an available Hex kernel variant is requested for the operator (NKB_HEX_VARIANT)
+bool HexVariantRequested(const nkb_op *op, int *variant);
 // name of the kernel the operator launches (for reports)
 const char *KernelName(const nkb_op *op, bool gather);
 size_t GenericSmemBytes(const nkb_op *op, int elem_bytes);
