@@ -1021,13 +1021,11 @@ extern "C" int nkb_sys_create(const nkb_sys_desc *desc, nkb_sys **out)
         !salloc((void **)&sh->d_aidx, nloc * sizeof(int)) ||
         (desc->sign && !salloc((void **)&sh->d_sign, nloc * sizeof(double))))
         return SetError(NKB_ERR_NOMEM, "nkb_sys_create: device allocation of the map failed");
-    NKB_CUDA_TRY(cudaMemcpy(sh->d_map, desc->map, nloc * sizeof(int), cudaMemcpyHostToDevice));
-    NKB_CUDA_TRY(cudaMemcpy(sh->d_aptr, aptr.data(), (sh->nglob + 1) * sizeof(int),
-                            cudaMemcpyHostToDevice));
-    NKB_CUDA_TRY(cudaMemcpy(sh->d_aidx, aidx.data(), nloc * sizeof(int), cudaMemcpyHostToDevice));
+    NKB_CUDA_TRY(CopyIn(sh->d_map, desc->map, nloc * sizeof(int)));
+    NKB_CUDA_TRY(CopyIn(sh->d_aptr, aptr.data(), (sh->nglob + 1) * sizeof(int)));
+    NKB_CUDA_TRY(CopyIn(sh->d_aidx, aidx.data(), nloc * sizeof(int)));
     if (desc->sign)
-        NKB_CUDA_TRY(cudaMemcpy(sh->d_sign, desc->sign, nloc * sizeof(double),
-                                cudaMemcpyHostToDevice));
+        NKB_CUDA_TRY(CopyIn(sh->d_sign, desc->sign, nloc * sizeof(double)));
 
     nkb_sys *S = new nkb_sys();
     S->sh      = sh;
@@ -1183,11 +1181,10 @@ extern "C" int nkb_sys_set_blocks(nkb_sys *S, int nblk, const int *bptr, const i
         release();
         return SetError(NKB_ERR_NOMEM, "nkb_sys_set_blocks: %ld doubles of blocks", tot);
     }
-    if (cudaMemcpy(dp, bptr, (nblk + 1) * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(di, bidx, nidx * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(dof, boff.data(), nblk * sizeof(long), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(dm, binv, tot * sizeof(double), cudaMemcpyDefault) != cudaSuccess ||
-        cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) // binv may be device memory
+    if (CopyIn(dp, bptr, (nblk + 1) * sizeof(int)) != cudaSuccess ||
+        CopyIn(di, bidx, nidx * sizeof(int)) != cudaSuccess ||
+        CopyIn(dof, boff.data(), nblk * sizeof(long)) != cudaSuccess ||
+        CopyIn(dm, binv, tot * sizeof(double)) != cudaSuccess) // binv may be device memory
     {
         release();
         return SetError(NKB_ERR_CUDA, "nkb_sys_set_blocks: upload");
@@ -1749,7 +1746,7 @@ extern "C" int nkb_sys_profile_iteration(nkb_sys *S, int iters, nkb_sys_profile 
     CGState run = h;
     run.done    = 0;
     run.maxit   = 1 << 30;
-    NKB_CUDA_TRY(cudaMemcpy(S->st, &run, sizeof(run), cudaMemcpyHostToDevice));
+    NKB_CUDA_TRY(CopyIn(S->st, &run, sizeof(run)));
     int rc = NKB_OK;
     NKB_CUDA_TRY(cudaEventRecord(e[0], s));
     for (int it = 0; it < iters && !rc; ++it)
@@ -1764,7 +1761,7 @@ extern "C" int nkb_sys_profile_iteration(nkb_sys *S, int iters, nkb_sys_profile 
     CGState zero = run;
     zero.alpha = zero.beta = 0.0;
     NKB_CUDA_TRY(cudaStreamSynchronize(s));
-    NKB_CUDA_TRY(cudaMemcpy(S->st, &zero, sizeof(zero), cudaMemcpyHostToDevice));
+    NKB_CUDA_TRY(CopyIn(S->st, &zero, sizeof(zero)));
     NKB_CUDA_TRY(cudaEventRecord(e[2], s));
     for (int it = 0; it < iters; ++it)
         k_update<double><<<nbU, kRedThreads, 0, s>>>(S->nn, S->ndir, S->st, S->p, S->q, S->x,
@@ -1790,7 +1787,7 @@ extern "C" int nkb_sys_profile_iteration(nkb_sys *S, int iters, nkb_sys_profile 
     cudaEventDestroy(e4);
     cudaEventDestroy(e5);
     // restore the state of the last solve
-    NKB_CUDA_TRY(cudaMemcpy(S->st, &h, sizeof(h), cudaMemcpyHostToDevice));
+    NKB_CUDA_TRY(CopyIn(S->st, &h, sizeof(h)));
     if (rc)
         return rc;
     prof->op_ms       = t01 / iters;

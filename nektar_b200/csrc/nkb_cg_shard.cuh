@@ -385,7 +385,7 @@ static int UploadPlan(ShardDev &d, const nkb_shard_plan &p, int ndir)
         if (!bytes)
             return true;
         return cudaMalloc(dst, bytes) == cudaSuccess &&
-               cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
+               CopyIn(*dst, src, bytes) == cudaSuccess;
     };
     d.rank    = p.rank;
     d.nint    = p.nint;

@@ -142,7 +142,7 @@ extern "C" int nkb_op_create_dense_rect(int rows, int cols, int nelmt, const dou
         cudaEventCreate(&op->ev0) != cudaSuccess || cudaEventCreate(&op->ev1) != cudaSuccess)
         return fail(SetError(NKB_ERR_CUDA, "nkb_op_create_dense: stream/event creation failed"));
     if (cudaMalloc(&op->d_err, 2 * sizeof(int)) != cudaSuccess ||
-        cudaMemset(op->d_err, 0, 2 * sizeof(int)) != cudaSuccess)
+        ClearMemory(op->d_err, 2 * sizeof(int)) != cudaSuccess)
         return fail(SetError(NKB_ERR_CUDA, "nkb_op_create_dense: error word"));
     const size_t bytes = size_t(nelmt) * rows * cols * sizeof(double);
     if (bytes)
@@ -150,10 +150,7 @@ extern "C" int nkb_op_create_dense_rect(int rows, int cols, int nelmt, const dou
         if (cudaMalloc(&op->geo, bytes) != cudaSuccess)
             return fail(SetError(NKB_ERR_NOMEM, "nkb_op_create_dense: %zu bytes of blocks", bytes));
         // host or device blocks (unified addressing tells them apart)
-        // a copy from device memory does not wait for itself: finished here,
-        // so the caller may free the source on return
-        if (cudaMemcpy(op->geo, mats, bytes, cudaMemcpyDefault) != cudaSuccess ||
-            cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess)
+        if (CopyIn(op->geo, mats, bytes) != cudaSuccess)
             return fail(SetError(NKB_ERR_CUDA, "nkb_op_create_dense: upload"));
     }
     *out = op;

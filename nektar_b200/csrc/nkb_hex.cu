@@ -132,8 +132,7 @@ int BuildTcTables(nkb_op *op)
     op->tc_tab = nullptr;
     if (cudaMalloc(&op->tc_tab, img.size() * sizeof(float)) != cudaSuccess)
         return SetError(NKB_ERR_NOMEM, "tensor-core Hex tables");
-    NKB_CUDA_TRY(cudaMemcpy(op->tc_tab, img.data(), img.size() * sizeof(float),
-                            cudaMemcpyHostToDevice));
+    NKB_CUDA_TRY(CopyIn(op->tc_tab, img.data(), img.size() * sizeof(float)));
     op->tc_bytes = int(img.size() * sizeof(float));
     return NKB_OK;
 }

@@ -1223,7 +1223,7 @@ template <int SHAPE, int NM, int NQ, int OP, typename T> int LineBuildAux(nkb_op
     std::memcpy(image.data() + nr, words.data(), nw);
     op->line_words = nr;
     NKB_CUDA_TRY(cudaMalloc(&op->line_aux, image.size()));
-    NKB_CUDA_TRY(cudaMemcpy(op->line_aux, image.data(), image.size(), cudaMemcpyHostToDevice));
+    NKB_CUDA_TRY(CopyIn(op->line_aux, image.data(), image.size()));
     return NKB_OK;
 }
 

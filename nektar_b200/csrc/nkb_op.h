@@ -77,6 +77,11 @@ template <typename T>
 int LaunchGeneric3(const nkb_op *op, const T *in, const T *in1, const T *in2, T *o0, T *o1, T *o2,
                    const int *gmap, const double *gsign, cudaStream_t s,
                    const int *skip = nullptr, const double *lambda = nullptr);
+// copies (or clears) n bytes of set-up data, in host or device memory, and returns once
+// they are there: cudaMemcpy may return before a pageable copy has arrived, and the
+// streams that the operators and systems run on are not ordered after the legacy stream
+cudaError_t CopyIn(void *dst, const void *src, size_t n);
+cudaError_t ClearMemory(void *dst, size_t n);
 // line kernels (nkb_line.cu). LineSetup decides whether the operator runs on
 // them and prepares its tables and layout (before the geometry is packed);
 // LaunchLine launches the one that was set up

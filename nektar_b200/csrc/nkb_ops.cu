@@ -596,6 +596,20 @@ static int Repack(nkb_op *op)
     return NKB_OK;
 }
 
+cudaError_t CopyIn(void *dst, const void *src, size_t n)
+{
+    if (n == 0)
+        return cudaSuccess;
+    const cudaError_t e = cudaMemcpy(dst, src, n, cudaMemcpyDefault);
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
+cudaError_t ClearMemory(void *dst, size_t n)
+{
+    const cudaError_t e = cudaMemset(dst, 0, n);
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 // a device copy of n doubles given in host or device memory (FP64: copied as
 // they are; FP32: converted on the host)
 template <typename T> static int Upload(T **dst, const double *src, size_t n)
@@ -603,18 +617,14 @@ template <typename T> static int Upload(T **dst, const double *src, size_t n)
     NKB_CUDA_TRY(cudaMalloc(dst, n * sizeof(T)));
     if constexpr (std::is_same_v<T, double>)
     {
-        // a copy from device memory does not wait for itself: finish it
-        // before the pack (on the operator's own stream) reads it and the
-        // caller frees the source
-        NKB_CUDA_TRY(cudaMemcpy(*dst, src, n * sizeof(T), cudaMemcpyDefault));
-        NKB_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+        NKB_CUDA_TRY(CopyIn(*dst, src, n * sizeof(T)));
     }
     else
     {
         std::vector<T> tmp(n);
         for (size_t i = 0; i < n; ++i)
             tmp[i] = T(src[i]);
-        NKB_CUDA_TRY(cudaMemcpy(*dst, tmp.data(), n * sizeof(T), cudaMemcpyHostToDevice));
+        NKB_CUDA_TRY(CopyIn(*dst, tmp.data(), n * sizeof(T)));
     }
     return NKB_OK;
 }
@@ -739,7 +749,7 @@ extern "C" int nkb_op_create(const nkb_op_desc *desc, nkb_op **out)
         cudaEventCreate(&op->ev0) != cudaSuccess || cudaEventCreate(&op->ev1) != cudaSuccess)
         return fail(SetError(NKB_ERR_CUDA, "nkb_op_create: stream/event creation failed"));
     if (cudaMalloc(&op->d_err, 2 * sizeof(int)) != cudaSuccess ||
-        cudaMemset(op->d_err, 0, 2 * sizeof(int)) != cudaSuccess)
+        ClearMemory(op->d_err, 2 * sizeof(int)) != cudaSuccess)
         return fail(SetError(NKB_ERR_CUDA, "nkb_op_create: error word"));
 
     // 1-D tables
@@ -991,7 +1001,7 @@ int CheckOpError(nkb_op *op)
     NKB_CUDA_TRY(cudaMemcpy(&word, op->d_err, sizeof(int), cudaMemcpyDeviceToHost));
     if (!word)
         return NKB_OK;
-    NKB_CUDA_TRY(cudaMemset(op->d_err, 0, sizeof(int)));
+    NKB_CUDA_TRY(ClearMemory(op->d_err, sizeof(int)));
     return SetError(NKB_ERR_TIMEOUT,
                     "operator kernel: a bounded wait for the geometry copy gave up (code %d); the "
                     "outputs of the elements it guarded were not written",
@@ -1017,7 +1027,7 @@ extern "C" int nkb_op_set_wait_limit(nkb_op *op, int polls)
         return SetError(NKB_ERR_INVALID, "nkb_op_set_wait_limit: %d polls (at most 2^24 - 1)", polls);
     NKB_CUDA_TRY(cudaSetDevice(op->device));
     const int word = polls < 0 ? 0 : polls + 1;
-    NKB_CUDA_TRY(cudaMemcpy(op->d_err + 1, &word, sizeof(int), cudaMemcpyHostToDevice));
+    NKB_CUDA_TRY(CopyIn(op->d_err + 1, &word, sizeof(int)));
     return NKB_OK;
 }
 

@@ -1,0 +1,76 @@
+"""The library's host code on a CUDA runtime that runs nothing (cpp/fake_cudart.cpp):
+faults that a GPU shows only now and then, or by ending the process."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from tests.helpers import ROOT
+
+SRC = os.path.join(ROOT, "tests", "cpp", "fake_cudart.cpp")
+SHAPES = ("hex", "prism", "tet")
+OPS = ("bwdtrans", "iproduct", "physderiv", "iproduct_deriv", "helmholtz", "linear_adr")
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    """The library's objects linked with the runtime's stand-in."""
+    from nektar_b200 import build
+    objs = [os.path.join(build.BUILD, s + ".o") for s in build.SOURCES]
+    if not all(os.path.exists(o) for o in objs):
+        pytest.skip("the objects of the build are not here")
+    out = str(tmp_path_factory.mktemp("fake") / "libnekb200_fake.so")
+    inc = os.path.join(os.path.dirname(os.path.dirname(build._nvcc())), "include")
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic",
+                           "-I" + inc, SRC] + objs + ["-ldl", "-o", out])
+    return out
+
+
+def run(lib, body, **env):
+    """body in a process of its own, with nb, np, lib and mesh(shape, nm, n) defined."""
+    head = ("import numpy as np\nimport nektar_b200 as nb\nfrom nektar_b200 import _capi as C\n"
+            "C.LIB_PATH = %r\nlib = C.lib()\n"
+            "SHAPES, OPS = %r, %r\n"
+            "def mesh(shape, nm, n=1, amp=0.05):\n"
+            "    return nb.BoxMesh(shape, n, nm, nm + 1, amp=amp)\n" % (lib, SHAPES, OPS))
+    p = subprocess.run([sys.executable, "-c", head + body], cwd=ROOT, capture_output=True,
+                       text=True, timeout=300, env=dict(os.environ, **env))
+    assert p.returncode == 0, (p.returncode, p.stderr[-3000:])
+
+
+@pytest.mark.parametrize("env", [{}, {"NKB_HEX_VARIANT": "5"}, {"NKB_KERNEL": "generic"}])
+def test_set_up_waits_for_its_copies(fake, env):
+    """Operators, systems and shards run on streams that the legacy stream does not
+    order: what their set-up copies and clears there has arrived when it returns, and
+    before any kernel of the set-up."""
+    run(fake, """
+for shape in SHAPES:
+    for name in OPS:
+        for precision in ("fp64", "fp32"):
+            for amp in (0.05, 0.0):
+                op = nb.Operator(name, mesh(shape, 5, 2, amp), precision=precision)
+                assert lib.fake_outstanding() == 0, (shape, name, precision, amp)
+m = mesh("hex", 4, 2)
+gmap, nglob, ndir = m.assembly()
+ops = [nb.Operator("helmholtz", m)]
+ops32 = [nb.Operator("helmholtz", m, precision="fp32")]
+S = nb.GlobalLinSys(ops, gmap, nglob, ndir, sign=np.ones(len(gmap)), ops32=ops32)
+assert lib.fake_outstanding() == 0
+ops[0].set_wait_limit(4)
+assert lib.fake_outstanding() == 0
+S.set_blocks([(ndir + np.arange(3), np.eye(3))])
+assert lib.fake_outstanding() == 0
+S.profile(1)
+assert lib.fake_outstanding() == 0
+from nektar_b200.sharded import DeviceShardGroup, shard_plans
+plans = shard_plans(np.asarray(gmap), ndir, 2, nc=m.nc)
+nt = m.nt
+halves = [nb.Operator("helmholtz", shape="hex", nm=m.nm, nq=m.nq, nelmt=4, T=m.T,
+                      jac=m.jac[k:k + 4 * nt], df=np.ascontiguousarray(m.df[:, k:k + 4 * nt]),
+                      deformed=True) for k in (0, 4 * nt)]
+G = DeviceShardGroup(plans, [[o] for o in halves])
+assert lib.fake_outstanding() == 0
+assert lib.fake_early_launches() == 0
+assert lib.fake_launches() > 0
+""", **env)
