@@ -493,6 +493,8 @@ int LaunchGeneric3(const nkb_op *op, const T *in, const T *in1, const T *in2, T 
                    const int *gmap, const double *gsign, cudaStream_t s, const int *skip,
                    const double *lambda)
 {
+    if (op->nelmt == 0)
+        return NKB_OK; // nothing to launch, nor to spread over the SMs
     if (!op->line_tabs.empty())
         return LaunchLine<T>(op, in, in1, in2, o0, o1, o2, gmap, gsign, s, skip,
                              T(lambda ? *lambda : op->lambda));

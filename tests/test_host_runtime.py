@@ -74,3 +74,26 @@ assert lib.fake_outstanding() == 0
 assert lib.fake_early_launches() == 0
 assert lib.fake_launches() > 0
 """, **env)
+
+
+def test_an_empty_collection_launches_nothing(fake):
+    """Every operator over no elements, through every apply entry point."""
+    run(fake, """
+x = np.zeros(1)
+for shape in SHAPES:
+    m = mesh(shape, 5)
+    for name in OPS:
+        for precision in ("fp64", "fp32"):
+            op = nb.Operator(name, shape=shape, nm=5, nq=m.nq, nelmt=0, T=m.T, jac=m.jac[:0],
+                             df=np.ascontiguousarray(m.df[:, :0]), deformed=True,
+                             precision=precision)
+            before = lib.fake_launches()
+            p = x.ctypes.data
+            op.apply_device(p, p, p, p)
+            if precision == "fp64":
+                op(x[:0])
+                if name == "iproduct_deriv":
+                    op.apply3(x[:0], x[:0], x[:0])
+                    op.apply3_device(p, p, p, p)
+            assert lib.fake_launches() == before, (shape, name, precision)
+""")
