@@ -40,6 +40,7 @@ struct nkb_batch
     cudaGraphExec_t graph = nullptr;
     const void *g_in = nullptr;
     void *g_out = nullptr;
+    std::vector<double> g_lambda; // of every operator, at the capture
     double *stage = nullptr; // host-pointer staging (in + out)
     float last_ms = 0.f;
 };
@@ -79,12 +80,15 @@ template <typename T> int LaunchAll(nkb_batch *B, const T *in, T *out, cudaStrea
     }
     return NKB_OK;
 }
-// launch the batch's graph on `run`, capturing it first when (in, out)
-// changed; timed by ev0 / ev1
+// launch the batch's graph on `run`, capturing it first when (in, out) or
+// an operator's lambda changed (the launches carry them by value; diffusion
+// and velocities are read from the packed geometry); timed by ev0 / ev1
 template <typename T> int RunGraph(nkb_batch *B, const T *din, T *dout, cudaStream_t run)
 {
-    // one graph per (input, output) pair; re-captured when they change
-    if (!B->graph || B->g_in != din || B->g_out != dout)
+    const bool same_lambda =
+        std::equal(B->ops.begin(), B->ops.end(), B->g_lambda.begin(), B->g_lambda.end(),
+                   [](const nkb_op *op, double lambda) { return op->lambda == lambda; });
+    if (!B->graph || B->g_in != din || B->g_out != dout || !same_lambda)
     {
         if (B->graph)
             cudaGraphExecDestroy(B->graph);
@@ -107,6 +111,9 @@ template <typename T> int RunGraph(nkb_batch *B, const T *din, T *dout, cudaStre
             return SetError(NKB_ERR_CUDA, "nkb_batch_apply: instantiate: %s", cudaGetErrorString(ce));
         B->g_in  = din;
         B->g_out = dout;
+        B->g_lambda.clear();
+        for (const nkb_op *op : B->ops)
+            B->g_lambda.push_back(op->lambda);
     }
     NKB_CUDA_TRY(cudaEventRecord(B->ev0, run));
     NKB_CUDA_TRY(cudaGraphLaunch(B->graph, run));

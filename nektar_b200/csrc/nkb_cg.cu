@@ -674,6 +674,7 @@ struct nkb_sys
     CGState *h_st = nullptr; // pinned [3]: FP64 state, FP32 state, state to write
     cudaGraphExec_t graph = nullptr;
     int graph_k = 0;
+    std::vector<double> graph_lambda; // lambdas that the captured launches carry
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, evq = nullptr;
     double *stage = nullptr; // host-pointer staging (2*nloc)
     long launches = 0;       // kernels launched by the current solve
@@ -682,6 +683,7 @@ struct nkb_sys
     CGState *st32 = nullptr;
     cudaGraphExec_t graph32 = nullptr;
     int graph32_k = 0;
+    std::vector<double> graph32_lambda;
     size_t bytes = 0; // device bytes of this instance
     SolveCtx sv;
 };
@@ -692,6 +694,13 @@ namespace nkb
 static const double *LambdaOf(const nkb_sys *S)
 {
     return S->has_lambda ? &S->lambda : nullptr;
+}
+
+// the lambdas that a launch of the system's operators takes now
+static void AddLambdas(const nkb_sys *S, bool fp32, std::vector<double> &out)
+{
+    for (const nkb_op *op : fp32 ? S->ops32 : S->ops)
+        out.push_back(S->has_lambda ? S->lambda : op->lambda);
 }
 
 // y_loc = A x_loc over all collections; x given either as a local vector or
@@ -791,7 +800,9 @@ static int EnsureGraph(nkb_sys *S, bool fp32, cudaStream_t s, int K)
 {
     cudaGraphExec_t &ge = fp32 ? S->graph32 : S->graph;
     int &gk             = fp32 ? S->graph32_k : S->graph_k;
-    if (ge && gk == K)
+    std::vector<double> lambdas, &gl = fp32 ? S->graph32_lambda : S->graph_lambda;
+    AddLambdas(S, fp32, lambdas);
+    if (ge && gk == K && gl == lambdas)
         return NKB_OK;
     if (ge)
         cudaGraphExecDestroy(ge);
@@ -812,6 +823,7 @@ static int EnsureGraph(nkb_sys *S, bool fp32, cudaStream_t s, int K)
     if (ce != cudaSuccess)
         return SetError(NKB_ERR_CUDA, "CG graph instantiate: %s", cudaGetErrorString(ce));
     gk = K;
+    gl = lambdas;
     return NKB_OK;
 }
 
@@ -1120,7 +1132,6 @@ extern "C" int nkb_sys_set_lambda(nkb_sys *S, double lambda)
     NKB_CUDA_TRY(cudaStreamSynchronize(S->stream));
     S->lambda     = lambda;
     S->has_lambda = true;
-    DropGraphs(S); // the captured launches carry the old lambda
     return NKB_OK;
 }
 

@@ -130,6 +130,7 @@ struct nkb_shard_group
     double *gsums = nullptr, *tot = nullptr; // [shards][4], [4]
     cudaGraphExec_t graph = nullptr;
     int graph_k = 0;
+    std::vector<double> graph_lambda; // lambdas that the captured launches carry
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     CGState *h_st = nullptr; // pinned
     long launches = 0;
@@ -305,7 +306,10 @@ static int GroupIteration(nkb_shard_group *G)
 
 static int EnsureGroupGraph(nkb_shard_group *G, int K)
 {
-    if (G->graph && G->graph_k == K)
+    std::vector<double> lambdas;
+    for (const ShardDev &d : G->sh)
+        AddLambdas(d.S, false, lambdas);
+    if (G->graph && G->graph_k == K && G->graph_lambda == lambdas)
         return NKB_OK;
     if (G->graph)
         cudaGraphExecDestroy(G->graph);
@@ -326,7 +330,8 @@ static int EnsureGroupGraph(nkb_shard_group *G, int K)
     cudaGraphDestroy(g);
     if (ce != cudaSuccess)
         return SetError(NKB_ERR_CUDA, "sharded CG graph instantiate: %s", cudaGetErrorString(ce));
-    G->graph_k = K;
+    G->graph_k      = K;
+    G->graph_lambda = lambdas;
     return NKB_OK;
 }
 

@@ -80,3 +80,34 @@ def test_fp32_batch_equals_collection_by_collection(optype):
     with pytest.raises(nb.NektarB200Error):
         B(np.zeros(B.in_size))  # host FP64 entry point refuses an FP32 batch
     B.close()
+
+
+@pytest.mark.parametrize("optype", ["helmholtz", "linear_adr"])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_factors_changed_between_two_applies(optype, precision):
+    """The captured graph follows an operator's new lambda and diffusion, on the same
+    buffers, as the operators applied one by one do."""
+    import torch
+    mm = MixedMesh(n=4, ncells=(20, 20, 10), pmin=2, pmax=3, seed=4)
+    ops = [nb.Operator(optype, m, precision=precision) for m in mm.meshes()]
+    dt = torch.float64 if precision == "fp64" else torch.float32
+    B = nb.Batch(ops)
+    x = torch.rand(B.in_size, dtype=dt, device="cuda") * 2 - 1
+    y, ref = (torch.empty(B.out_size, dtype=dt, device="cuda") for _ in range(2))
+    s = torch.cuda.current_stream().cuda_stream
+    for step, lam in enumerate((1.5, 0.25, 7.0)):
+        for k, op in enumerate(ops):
+            if step == 1 and k:
+                continue  # one operator's lambda alone
+            if optype == "helmholtz" and step == 2:
+                op.set_factors(lam, nb.DIFF_CONST, [1.5, 0.2, 0.8, -0.1, 0.3, 1.1])
+            else:
+                op.set_factors(lam)
+        B.apply_device(x.data_ptr(), y.data_ptr(), stream=s)
+        o = 0
+        for op in ops:
+            op.apply_device(x[o:].data_ptr(), ref[o:].data_ptr(), stream=s)
+            o += op.in_size
+        torch.cuda.synchronize()
+        assert torch.equal(y, ref), (step, lam)
+    B.close()

@@ -178,3 +178,31 @@ def test_all_dirichlet_system_returns_the_dirichlet_values():
     op.close()
     assert rep.converged and rep.iterations == 0
     assert np.array_equal(x, x0)
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_cg_graph_follows_the_operators_factors(mixed):
+    """A lambda given to the operators after a solve reaches the next one's captured
+    iterations: the same bits as with direct launches, and the new system's solution."""
+    m = nb.BoxMesh("hex", 3, 4, 5, amp=0.05)
+    gmap, nglob, ndir = m.assembly()
+    b = np.random.default_rng(8).uniform(-1, 1, m.nelmt * m.nc)
+
+    def ops(lam):
+        pair = [nb.Operator("helmholtz", m), nb.Operator("helmholtz", m, precision="fp32")]
+        for op in pair:
+            op.set_factors(lam)
+        return pair
+
+    pair = ops(1.0)
+    S = nb.GlobalLinSys(pair[:1], gmap, nglob, ndir, ops32=pair[1:])
+    S.solve(b, tol=1e-11, mixed=mixed)
+    for op in pair:
+        op.set_factors(400.0)
+    x, rep = S.solve(b, tol=1e-11, mixed=mixed)
+    fresh = nb.GlobalLinSys(ops(400.0)[:1], gmap, nglob, ndir)
+    y, _ = fresh.solve(b, tol=1e-11)
+    assert rep.converged and rel_l2(x, y) < 1e-9
+    if not mixed:  # the mixed solve always runs captured iterations
+        z, direct = S.solve(b, tol=1e-11, use_graph=False)
+        assert np.array_equal(x, z) and rep.iterations == direct.iterations

@@ -135,3 +135,23 @@ def test_a_shard_solves_only_through_its_group():
     assert nb.lib().nkb_shard_group_create(hs, G._cp, 2, None, ctypes.byref(g2)) == \
         nb.C.NKB_ERR_INVALID
     G.close()
+
+
+def test_shards_follow_a_new_lambda():
+    """A lambda set on the shards between two solves reaches the group's captured
+    iterations."""
+    from nektar_b200.sharded import DeviceShardGroup, shard_plans
+    m, gmap, nglob, ndir, b, x0 = _problem()
+    nc = m.nc
+    plans = shard_plans(gmap, ndir, 2, nc=nc)
+    G = DeviceShardGroup(plans, [_ops(m, p["lo"], p["hi"]) for p in plans])
+    bs, xs = ([v[p["lo"] * nc:p["hi"] * nc] for p in plans] for v in (b, x0))
+    G.solve(bs, xs, tol=1e-11)
+    for S in G.systems:
+        S.set_lambda(400.0)
+    x, reps = G.solve(bs, xs, tol=1e-11)
+    G.close()
+    op = _ops(m, 0, m.nelmt)
+    op[0].set_factors(400.0)
+    y, _ = nb.GlobalLinSys(op, gmap, nglob, ndir).solve(b, x0, tol=1e-11)
+    assert all(r.converged for r in reps) and rel_l2(np.concatenate(x), y) < 1e-9
