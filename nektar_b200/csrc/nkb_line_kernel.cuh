@@ -23,6 +23,13 @@
 // Straight-sided elements have one Jacobian and one set of derivative
 // factors: 16 values per element (geoc), the weights and collapsed-coordinate
 // factors being products of 1-D tables, instead of 1 to 10 values per point.
+// FP32 operators apply them in FP64 and round the results, or (Helmholtz,
+// LinearADR) read factors per point that were formed in FP64 and rounded once:
+// formed in FP32 they put results up to 11 % further from the FP64 ones (tet
+// LinearADR, 4 modes). Of the two, FP64 arithmetic is the quicker where a point
+// takes nine factors (IProductWRTDerivBase, tet 8 modes x 37202: 206 us, factors
+// 229; in FP32 235), factors where it takes seven or ten (Helmholtz, prism 7 modes
+// x 47831: 204, FP64 219, in FP32 200; tets of 8 modes alone 284, 245 and 221).
 //
 // The collapsed-vertex and singular-edge terms of BwdTransKernels.hpp:231-403
 // and IProductKernels.hpp:355-655 are folded into the first stage: with A_p,
@@ -241,6 +248,9 @@ template <int SHAPE, int NM, int NQ, int OP, typename T> struct LineDims
                                                    : NM * (NM + 1) * (NM + 2) / 6;
     static constexpr int XR = SHAPE == NKB_HEX ? NM | 1 : 1; // coefficient row stride
     static constexpr int XSIZE = SHAPE == NKB_HEX ? NM * NM * XR : NC;
+    // straight-sided elements too read a value per point, formed in FP64 and rounded
+    // once (nkb_ops.cu allocates no geoc then)
+    static constexpr bool PACKED = (OP == LN_HELM || OP == LN_ADR) && sizeof(T) == 4;
     static constexpr int NCUBE = OP == LN_IP ? 1 : (OP == LN_BWD ? 2 : 3);
     // threads: one per line of the direction with the most lines
     static constexpr int LA = K1 * K2, LB = K0 * K2, LC = K0 * K1;
@@ -407,6 +417,7 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
     constexpr bool VAR = L::VAR;
     constexpr bool HEX = SHAPE == NKB_HEX, TET = SHAPE == NKB_TET;
     constexpr bool HELM = OP == LN_HELM || OP == LN_ADR;
+    constexpr bool PACKED = L::PACKED;
     constexpr bool FROM_COEFFS = HELM || OP == LN_BWD, TO_COEFFS = OP != LN_BWD && OP != LN_PD;
     extern __shared__ __align__(128) unsigned char line_raw[];
     T *S0 = reinterpret_cast<T *>(line_raw);
@@ -417,7 +428,7 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
     const int tid = threadIdx.x;
     if (ne <= 0 || (a.skip && *a.skip))
         return;
-    const bool curved = a.geoc == nullptr;
+    const bool curved = PACKED || a.geoc == nullptr;
     const int nm      = VAR ? a.nm : NM, nm2 = nm * nm, np = nm * (nm + 1) / 2;
     const int nc      = HEX ? nm2 * nm : (TET ? nm * (nm + 1) * (nm + 2) / 6 : nm * np);
     if ((HELM || OP == LN_IPD || OP == LN_PD) && tid == 0 && curved)
@@ -684,10 +695,11 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
         // mesh's directions
         auto point = [&](long e, int n, int m0, int m1, int m2, T &v0, T &v1, T &v2) {
             // the packing's order of products
-            const T W = curved ? T(0) : T(a.geoc[e * kGeoc] * c.w0[m0] * c.w1[m1] * c.w2[m2]);
+            const double W =
+                curved ? 0.0 : a.geoc[e * kGeoc] * c.w0[m0] * c.w1[m1] * c.w2[m2];
             if (OP == LN_IP)
             {
-                v0 = a.in[e * NT + n] * (curved ? a.geo[e * a.gstride + n] : W);
+                v0 = a.in[e * NT + n] * (curved ? a.geo[e * a.gstride + n] : T(W));
                 return;
             }
             const T f0 = a.in[e * NT + n], f1 = a.in1[e * NT + n], f2 = a.in2[e * NT + n];
@@ -699,15 +711,13 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
                 v2         = fma(P[8 * NT], f2, fma(P[7 * NT], f1, P[6 * NT] * f0));
                 return;
             }
-            T P[kGeoc];
-#pragma unroll
-            for (int m = 7; m < kGeoc; ++m)
-                P[m] = T(a.geoc[e * kGeoc + m]);
-            v0 = W * fma(P[13], f2, fma(P[10], f1, P[7] * f0));
-            v1 = W * fma(P[14], f2, fma(P[11], f1, P[8] * f0));
-            v2 = W * fma(P[15], f2, fma(P[12], f1, P[9] * f0));
-            LineChainT<SHAPE>(T(c.h0[m0]), T(c.h1[m1]), T(c.g2[m2]), T(c.g1[m1] * c.g2[m2]), v0, v1,
-                              v2);
+            // in FP64 for FP32 fields too, so that nothing is rounded but the results
+            const double *P = a.geoc + e * kGeoc, d0 = f0, d1 = f1, d2 = f2;
+            double x0 = W * fma(P[13], d2, fma(P[10], d1, P[7] * d0));
+            double x1 = W * fma(P[14], d2, fma(P[11], d1, P[8] * d0));
+            double x2 = W * fma(P[15], d2, fma(P[12], d1, P[9] * d0));
+            LineChainT<SHAPE>(c.h0[m0], c.h1[m1], c.g2[m2], c.g1[m1] * c.g2[m2], x0, x1, x2);
+            v0 = T(x0), v1 = T(x1), v2 = T(x2);
         };
         if constexpr (L::REV)
         {
@@ -858,14 +868,14 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
                     g0[i] = fma(G02, q2, fma(G01, q1, __ldg(Gi + C00 * NT) * q0));
                 }
             }
-            else
+            else if constexpr (!PACKED)
             {
                 const double *P = a.geoc + (e0 + re) * kGeoc;
-                const T J = T(P[0]), G00 = T(P[1]), G11 = T(P[2]), G22 = T(P[3]), G01 = T(P[4]),
-                        G02 = T(P[5]), G12 = T(P[6]);
-                const double ww = HEX ? c.w0[rk] * c.w1[rj] : c.w1[rj] * c.w2[rk];
-                const T h1 = T(c.h1[rj]), g2 = HEX ? T(0) : T(c.g2[rk]),
-                        g12 = HEX ? T(0) : T(c.g1[rj] * c.g2[rk]);
+                const T J = P[0], G00 = P[1], G11 = P[2], G22 = P[3], G01 = P[4], G02 = P[5],
+                        G12 = P[6];
+                const T ww = HEX ? c.w0[rk] * c.w1[rj] : c.w1[rj] * c.w2[rk];
+                const T h1 = c.h1[rj], g2 = HEX ? 0.0 : c.g2[rk],
+                        g12 = HEX ? 0.0 : c.g1[rj] * c.g2[rk];
                 const T *V = OP == LN_ADR ? a.geo + rgeo + 7 * NT : nullptr;
 #pragma unroll
                 for (int i = 0; i < K0; ++i)
@@ -873,7 +883,7 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
                     const int s = rbase + i * PS;
                     // in the mesh's directions
                     T q0 = HEX ? S2[s] : g0[i], q1 = S1[s], q2 = HEX ? g0[i] : S2[s];
-                    const T W = T(ww * (HEX ? c.w2[HEX ? i : 0] : c.w0[i]));
+                    const T W = ww * (HEX ? c.w2[HEX ? i : 0] : c.w0[i]);
                     T mass    = W * J * u[i];
                     if (OP == LN_ADR)
                         mass = fma(__ldg(V + 2 * NT + i * L::LA), q2,

@@ -790,7 +790,10 @@ extern "C" int nkb_op_create(const nkb_op_desc *desc, nkb_op **out)
         return fail(rc);
     if (op->ncomp && op->nelmt)
     {
-        const bool straight = !op->line_tabs.empty() && !op->deformed;
+        // 16 values per straight-sided element on the line kernels, but for FP32
+        // Helmholtz and LinearADR (nkb_line_kernel.cuh, PACKED)
+        const bool straight = !op->line_tabs.empty() && !op->deformed &&
+                              !(helm_like && op->precision == NKB_FP32);
         const size_t nc16   = size_t(op->nelmt) * 16;
         if (straight && cudaMalloc(&op->geoc, nc16 * sizeof(double)) != cudaSuccess)
             return fail(SetError(NKB_ERR_NOMEM, "nkb_op_create: geometry (%zu doubles)", nc16));

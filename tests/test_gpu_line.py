@@ -97,3 +97,49 @@ def test_line_kernel_three_input_fields_and_infinities():
     bad = ~torch.isfinite(y.view(m.nelmt, m.nc)).all(1)
     assert torch.equal(y.view(torch.int64), z.view(torch.int64))
     assert bad.nonzero().ravel().tolist() == [5]
+
+
+def _pointwise(m, name, precision, scale=1.0):
+    """The operator of m's straight-sided elements, and of the same elements given point
+    by point as curved ones are; lengths scaled by `scale`."""
+    rng = np.random.default_rng(m.nm)
+    jac, df = m.jac * scale ** 3, m.df / scale
+    vel = rng.uniform(-1, 1, (3, m.nelmt * m.nt))
+    ops = []
+    for deformed in (False, True):
+        g = (np.repeat(jac, m.nt), np.repeat(df, m.nt, axis=1)) if deformed else (jac, df)
+        op = nb.Operator(name, shape=m.shape, nm=m.nm, nq=m.nq, nelmt=m.nelmt, T=m.T, jac=g[0],
+                         df=np.ascontiguousarray(g[1]), deformed=deformed, precision=precision)
+        if name in ("helmholtz", "linear_adr"):
+            op.set_factors(0.7)
+        if name == "linear_adr":
+            op.set_varcoeffs(*vel)
+        ops.append(op)
+    return ops
+
+
+@pytest.mark.parametrize("name", ["helmholtz", "linear_adr"])
+@pytest.mark.parametrize("nm,nq", [(2, 3), (4, 5), (5, 9), (8, 9), (11, 12)])
+@pytest.mark.parametrize("shape", ["hex", "prism", "tet"])
+def test_fp32_straight_sided_factors_are_rounded_once(shape, nm, nq, name):
+    """FP32 operators on straight-sided elements use factors formed in FP64 and rounded
+    once at each point: the bits of the same elements given point by point."""
+    import torch
+    m = nb.BoxMesh(shape, 2, nm, nq)
+    assert not m.deformed
+    straight, curved = _pointwise(m, name, "fp32")
+    x = np.random.default_rng(nq).uniform(-1, 1, straight.in_size)
+    assert np.array_equal(_apply(straight, x, torch.float32), _apply(curved, x, torch.float32))
+
+
+@pytest.mark.parametrize("nm,nq", [(3, 4), (6, 7), (5, 9)])
+@pytest.mark.parametrize("shape", ["hex", "prism", "tet"])
+def test_fp32_straight_sided_metric_is_formed_in_fp64(shape, nm, nq):
+    """IProductWRTDerivBase on elements whose Jacobian and weights (1e-45 and below)
+    have no FP32 value, although their products with the derivative factors do."""
+    import torch
+    m = nb.BoxMesh(shape, 2, nm, nq)
+    x = np.random.default_rng(nq).uniform(-1, 1, 3 * m.nelmt * m.nt)
+    y = _apply(_pointwise(m, "iproduct_deriv", "fp32", 1e-14)[0], x, torch.float32)
+    z = _apply(_pointwise(m, "iproduct_deriv", "fp64", 1e-14)[0], x, torch.float64)
+    assert rel_l2(y, z) < TOL["fp32"]
