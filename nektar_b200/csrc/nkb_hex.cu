@@ -24,21 +24,6 @@ namespace nkb
 
 // NKB_KERNEL=generic selects the shape-generic kernels for every operator
 // (used to test both implementations against each other).
-int SmCount(int device)
-{
-    static int counts[64] = {0};
-    if (device < 0 || device >= 64)
-        return 148;
-    if (counts[device] == 0)
-    {
-        int n = 0;
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0)
-            n = 148;
-        counts[device] = n;
-    }
-    return counts[device];
-}
-
 static bool ForceGeneric()
 {
     const char *v = std::getenv("NKB_KERNEL");

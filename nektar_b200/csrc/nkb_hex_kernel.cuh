@@ -16,7 +16,6 @@
 namespace nkb
 {
 
-int SmCount(int device); // multiprocessors of a device (nkb_hex.cu)
 
 
 template <typename T> struct HexArgs
@@ -529,7 +528,7 @@ static int HexTcLaunch(const nkb_op *op, const HexArgs<float> &a, bool gather, c
     // persistent grid: the CTAs per SM the launch bounds were built for
     // (shared and tensor memory allow that many; ncu confirms the register
     // limit), each walking its tiles
-    const long resident = long(Dm::MIN_CTAS) * SmCount(op->device);
+    const long resident = long(Dm::MIN_CTAS) * op->sms;
     const long nb       = ntile < resident ? ntile : resident;
     TcTables tt;
     tt.tab   = op->tc_tab;

@@ -65,8 +65,6 @@
 namespace nkb
 {
 
-int SmCount(int device); // multiprocessors of a device (nkb_hex.cu)
-
 enum
 {
     LN_BWD  = 0,
@@ -1256,7 +1254,7 @@ int LineOne(nkb_op *setup, const nkb_op *op, const LineArgs<T> *a, cudaStream_t 
     }
     // a collection smaller than one wave of full CTAs is spread over all SMs in
     // smaller ones (64 hexahedra of 4 modes: 6.5 us in 64 CTAs, 8.4 in 13)
-    const int slots   = SmCount(op->device) * L::MINB;
+    const int slots   = op->sms * L::MINB;
     LineArgs<T> run   = *a;
     run.epb           = std::min(L::EPB, (op->nelmt + slots - 1) / slots);
     const unsigned nb = unsigned((op->nelmt + run.epb - 1) / run.epb);

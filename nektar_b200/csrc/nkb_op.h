@@ -13,6 +13,7 @@ struct nkb_op
     int shape = 0, optype = 0, nm = 0, nq[3] = {0, 0, 0}, ptype[3] = {0, 0, 0};
     int nelmt = 0, deformed = 0, precision = 0, device = 0;
     int nc = 0, nt = 0, ncomp = 0;
+    int sms = 148; // multiprocessors of the device
     long gstride = 0; // packed geometry stride per element (multiple of 4 values)
 
     // 1-D tables on the device (FP64 and FP32 copies)

@@ -721,6 +721,10 @@ extern "C" int nkb_op_create(const nkb_op_desc *desc, nkb_op **out)
     op->deformed  = desc->deformed ? 1 : 0;
     op->precision = desc->precision;
     op->device    = desc->device;
+    if (cudaDeviceGetAttribute(&op->sms, cudaDevAttrMultiProcessorCount, op->device) !=
+            cudaSuccess ||
+        op->sms <= 0)
+        op->sms = 148;
     for (int d = 0; d < 3; ++d)
     {
         op->nq[d]    = nq[d];

@@ -97,3 +97,16 @@ for shape in SHAPES:
                     op.apply3_device(p, p, p, p)
             assert lib.fake_launches() == before, (shape, name, precision)
 """)
+
+
+def test_an_apply_asks_the_device_nothing(fake):
+    """What a launch needs to know of the device is read when the operator is created:
+    two threads' first applies share nothing that either of them writes."""
+    run(fake, """
+x = np.zeros(1)
+ops = [nb.Operator(name, mesh(shape, 4, 2)) for shape in SHAPES for name in OPS]
+before = lib.fake_attribute_queries()
+for op in ops:
+    op.apply_device(*4 * [x.ctypes.data])
+assert lib.fake_attribute_queries() == before
+""")
