@@ -17,7 +17,6 @@ namespace nkb
 {
 
 
-
 template <typename T> struct HexArgs
 {
     const T *in;

@@ -41,7 +41,7 @@ struct nkb_op
     // straight-sided element; tables and index words on the device
     std::vector<unsigned char> line_tabs;
     int geo_perm = 0;
-    double *geoc = nullptr;
+    double *geoc = nullptr; // begins, or lies behind geo in, the geometry's allocation
     void *line_aux    = nullptr;
     size_t line_words = 0; // offset of its words
 

@@ -553,7 +553,7 @@ template int LaunchGeneric<float>(const nkb_op *, const float *, float *, float 
                                   const int *, const double *, cudaStream_t, const int *,
                                   const double *);
 
-static int Repack(nkb_op *op)
+static PackArgs MakePackArgs(const nkb_op *op)
 {
     PackArgs a;
     std::memset(&a, 0, sizeof(a));
@@ -583,14 +583,23 @@ static int Repack(nkb_op *op)
     a.gstride = op->gstride;
     a.perm    = op->geo_perm;
     a.geoc    = op->geoc;
+    return a;
+}
+
+static void LaunchPack(const PackArgs &a, cudaStream_t s)
+{
+    const long tot = long(a.nelmt) * a.nt;
+    const int nb   = int(std::min<long>((tot + 255) / 256, 148L * 16));
+    k_pack<<<std::max(nb, 1), 256, 0, s>>>(a);
+}
+
+static int Repack(nkb_op *op)
+{
     if (op->ncomp == 0)
         return NKB_OK;
+    const PackArgs a = MakePackArgs(op);
     if (op->geo)
-    {
-        const long tot = long(op->nelmt) * op->nt;
-        const int nb   = int(std::min<long>((tot + 255) / 256, 148L * 16));
-        k_pack<<<std::max(nb, 1), 256, 0, op->stream>>>(a);
-    }
+        LaunchPack(a, op->stream);
     if (op->geoc)
         k_pack_straight<<<(op->nelmt + 127) / 128, 128, 0, op->stream>>>(a);
     NKB_CUDA_TRY(cudaGetLastError());
@@ -798,14 +807,17 @@ extern "C" int nkb_op_create(const nkb_op_desc *desc, nkb_op **out)
         // Helmholtz and LinearADR (nkb_line_kernel.cuh, PACKED)
         const bool straight = !op->line_tabs.empty() && !op->deformed &&
                               !(helm_like && op->precision == NKB_FP32);
-        const size_t nc16   = size_t(op->nelmt) * 16;
-        if (straight && cudaMalloc(&op->geoc, nc16 * sizeof(double)) != cudaSuccess)
-            return fail(SetError(NKB_ERR_NOMEM, "nkb_op_create: geometry (%zu doubles)", nc16));
+        const size_t nc16   = straight ? size_t(op->nelmt) * 16 : 0;
         // values per point: straight-sided elements on the line kernels need
-        // them only for LinearADR's velocities and Helmholtz's diagonal
-        const size_t n = straight && !helm_like ? 0 : size_t(op->nelmt) * op->gstride;
-        if (n && cudaMalloc(&op->geo, n * sizeof(double)) != cudaSuccess)
-            return fail(SetError(NKB_ERR_NOMEM, "nkb_op_create: geometry (%zu doubles)", n));
+        // them only for LinearADR's velocities (HelmholtzDiag packs its own).
+        // Both in one allocation, which geo, or else geoc, begins
+        const size_t n =
+            straight && opt != NKB_LINEAR_ADR ? 0 : size_t(op->nelmt) * op->gstride;
+        double *mem = nullptr;
+        if (cudaMalloc(&mem, (n + nc16) * sizeof(double)) != cudaSuccess)
+            return fail(SetError(NKB_ERR_NOMEM, "nkb_op_create: geometry (%zu doubles)", n + nc16));
+        op->geo  = n ? mem : nullptr;
+        op->geoc = straight ? mem + n : nullptr;
         if (n && op->precision == NKB_FP32 && cudaMalloc(&op->geo32, n * sizeof(float)) != cudaSuccess)
             return fail(SetError(NKB_ERR_NOMEM, "nkb_op_create: FP32 geometry"));
         if ((rc = Repack(op)))
@@ -1171,7 +1183,8 @@ extern "C" int nkb_op_last_kernel_ms(const nkb_op *op, float *ms)
 
 namespace nkb
 {
-static int HexDiag(const nkb_op *op, double *d_out, cudaStream_t s, double *d_stiff)
+static int HexDiag(const nkb_op *op, const double *geo, double *d_out, cudaStream_t s,
+                   double *d_stiff)
 {
     const int nm = op->nm, nq = op->nq[0];
     const size_t tn = size_t(nm) * nq;
@@ -1202,7 +1215,7 @@ static int HexDiag(const nkb_op *op, double *d_out, cudaStream_t s, double *d_st
                                           int(smem));
     if (ce == cudaSuccess && op->nelmt > 0)
     {
-        k_hex_diag<<<op->nelmt, threads, smem, s>>>(nm, nq, dtab, op->geo, op->gstride, op->nelmt,
+        k_hex_diag<<<op->nelmt, threads, smem, s>>>(nm, nq, dtab, geo, op->gstride, op->nelmt,
                                                     op->lambda, d_out, d_stiff);
         ce = cudaGetLastError();
     }
@@ -1214,18 +1227,15 @@ static int HexDiag(const nkb_op *op, double *d_out, cudaStream_t s, double *d_st
     return NKB_OK;
 }
 
-int HelmholtzDiag(const nkb_op *op, double *d_out, cudaStream_t s, double *d_stiff)
+static int DiagOf(const nkb_op *op, const double *geo, double *d_out, cudaStream_t s,
+                  double *d_stiff)
 {
-    if (op->optype == NKB_DENSE_BLOCK)
-        return DenseDiag(op, d_out, s, d_stiff);
-    if (op->optype != NKB_HELMHOLTZ)
-        return SetError(NKB_ERR_INVALID, "Helmholtz diagonal needs a Helmholtz operator");
     if (op->shape == NKB_HEX && op->nq[0] == op->nq[1] && op->nq[0] == op->nq[2])
-        return HexDiag(op, d_out, s, d_stiff);
+        return HexDiag(op, geo, d_out, s, d_stiff);
     GenArgs<double> a;
     a.d      = MakeDims(op);
     a.t      = MakeTabs<double>(op);
-    a.geo    = op->geo;
+    a.geo    = geo;
     a.lambda = op->lambda;
     a.in     = nullptr;
     a.out0   = d_out;
@@ -1247,6 +1257,25 @@ int HelmholtzDiag(const nkb_op *op, double *d_out, cudaStream_t s, double *d_sti
         kern<<<op->nelmt, threads, smem, s>>>(a, op->geo_perm);
     NKB_CUDA_TRY(cudaGetLastError());
     return NKB_OK;
+}
+
+int HelmholtzDiag(const nkb_op *op, double *d_out, cudaStream_t s, double *d_stiff)
+{
+    if (op->optype == NKB_DENSE_BLOCK)
+        return DenseDiag(op, d_out, s, d_stiff);
+    if (op->optype != NKB_HELMHOLTZ)
+        return SetError(NKB_ERR_INVALID, "Helmholtz diagonal needs a Helmholtz operator");
+    if (op->geo || op->nelmt == 0)
+        return DiagOf(op, op->geo, d_out, s, d_stiff);
+    // a straight-sided operator on the line kernels keeps no values per point
+    PackArgs a     = MakePackArgs(op);
+    const size_t n = size_t(op->nelmt) * op->gstride;
+    if (cudaMallocAsync((void **)&a.geo, n * sizeof(double), s) != cudaSuccess)
+        return SetError(NKB_ERR_NOMEM, "Helmholtz diagonal: geometry (%zu doubles)", n);
+    LaunchPack(a, s);
+    const int rc = DiagOf(op, a.geo, d_out, s, d_stiff);
+    NKB_CUDA_TRY(cudaFreeAsync(a.geo, s));
+    return rc;
 }
 } // namespace nkb
 
@@ -1295,9 +1324,8 @@ extern "C" void nkb_op_destroy(nkb_op *op)
     cudaFree(op->djac);
     cudaFree(op->ddf);
     cudaFree(op->dvel);
-    cudaFree(op->geo);
+    cudaFree(op->geo ? op->geo : op->geoc);
     cudaFree(op->geo32);
-    cudaFree(op->geoc);
     cudaFree(op->line_aux);
     cudaFree(op->scratch);
     cudaFree(op->d_err);

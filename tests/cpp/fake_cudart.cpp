@@ -18,7 +18,7 @@ struct Write
 };
 std::vector<Write> outstanding;
 int early_launches = 0, launches = 0, attribute_queries = 0;
-long next_handle = 0x1000;
+long next_handle = 0x1000, allocated = 0;
 
 bool Legacy(cudaStream_t s)
 {
@@ -55,6 +55,7 @@ extern "C" {
 int fake_outstanding() { return int(outstanding.size()); }
 int fake_early_launches() { return early_launches; }
 int fake_launches() { return launches; }
+long fake_allocated() { return allocated; }
 int fake_attribute_queries() { return attribute_queries; }
 
 void **__cudaRegisterFatBinary(void *) { return reinterpret_cast<void **>(&next_handle); }
@@ -104,7 +105,11 @@ cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "fake"; }
 cudaError_t cudaFuncSetAttribute(const void *, cudaFuncAttribute, int) { return cudaSuccess; }
 
-cudaError_t cudaMalloc(void **p, size_t n) { return *p = std::calloc(n + 1, 1), cudaSuccess; }
+cudaError_t cudaMalloc(void **p, size_t n)
+{
+    allocated += long(n);
+    return *p = std::calloc(n + 1, 1), cudaSuccess;
+}
 cudaError_t cudaFree(void *p) { return std::free(p), cudaSuccess; }
 cudaError_t cudaMallocAsync(void **p, size_t n, cudaStream_t) { return cudaMalloc(p, n); }
 cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return cudaFree(p); }

@@ -61,7 +61,7 @@ def test_line_and_generic_kernels_agree(monkeypatch, shape, nm, nq, amp, precisi
             assert rel_l2(y, z) < TOL[precision], (name, n, line.kernel())
 
 
-@pytest.mark.parametrize("shape", ["prism", "tet"])
+@pytest.mark.parametrize("shape", ["hex", "prism", "tet"])
 @pytest.mark.parametrize("amp", [0.05, 0.0])
 def test_line_kernel_diagonal_and_gather(monkeypatch, shape, amp):
     """The Helmholtz diagonal reads the line kernels' point order; a gathered

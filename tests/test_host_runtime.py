@@ -110,3 +110,20 @@ for op in ops:
     op.apply_device(*4 * [x.ctypes.data])
 assert lib.fake_attribute_queries() == before
 """)
+
+
+def test_straight_sided_operators_keep_no_values_per_point(fake):
+    """FP64 straight-sided operators hold 16 values per element; only LinearADR, whose
+    velocities vary, packs values per point."""
+    run(fake, """
+for shape in SHAPES:
+    for name in OPS:
+        sizes = []
+        for n in (2, 3):
+            m, before = mesh(shape, 8, n, amp=0.0), lib.fake_allocated()
+            op = nb.Operator(name, m)
+            sizes.append((lib.fake_allocated() - before, m.nelmt))
+        per_element = (sizes[1][0] - sizes[0][0]) / (sizes[1][1] - sizes[0][1]) / 8
+        # the caller's Jacobian and nine derivative factors, and the operator's values
+        assert per_element <= 10 + 16 + (10 * m.nt + 3 if name == "linear_adr" else 0), name
+""")
