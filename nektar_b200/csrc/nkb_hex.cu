@@ -283,12 +283,7 @@ const char *KernelName(const nkb_op *op, bool)
     if (op->optype == NKB_DENSE_BLOCK)
         return "k_dense_gemv (per-element dense blocks)";
     if (op->variant != kVariantHexHelm)
-    {
-        const bool helm = op->optype == NKB_HELMHOLTZ || op->optype == NKB_LINEAR_ADR;
-        if (helm && op->shape != NKB_HEX && !op->line_tabs.empty())
-            return "k_col_helm (Prism/Tet column kernel: k_line)";
         return op->line_tabs.empty() ? "k_generic" : "k_line (one thread per grid line)";
-    }
     return op->hex_variant == 5
                ? "k_hex_helm_tc (tcgen05 TF32 high/low tensor cores, FP32 accumulate)"
                : "k_hex_helm (TMA-staged geometry)";

@@ -169,14 +169,14 @@ def test_hex_kernel_variants_linear_adr_match_oracle(monkeypatch, n, nm, variant
 
 @pytest.mark.parametrize("shape,nm", [("prism", 3), ("prism", 7), ("prism", 11), ("tet", 4),
                                       ("tet", 8), ("tet", 11)])
-def test_column_kernel_linear_adr_matches_oracle(shape, nm):
+def test_line_kernel_linear_adr_matches_oracle(shape, nm):
     m = nb.BoxMesh(shape, 2, nm, nm + 1, amp=0.05)
     rng = np.random.default_rng(nm + 200)
     x = rng.uniform(-1, 1, m.nelmt * m.nc)
     vel = rng.uniform(-1, 1, 3 * m.nelmt * m.nt)
     k = m.nelmt * m.nt
     op = nb.Operator("linear_adr", m)
-    assert op.kernel().startswith("k_col_helm")
+    assert op.kernel().startswith("k_line")
     op.set_factors(-2.0)
     op.set_varcoeffs(vel[:k], vel[k:2 * k], vel[2 * k:])
     yo = O.linear_adr(shape, nm, m.nq, m.nelmt, _oracle_T(m), m.jac, m.df, -2.0, vel, x, True)

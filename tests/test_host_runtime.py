@@ -127,3 +127,13 @@ for shape in SHAPES:
         # the caller's Jacobian and nine derivative factors, and the operator's values
         assert per_element <= 10 + 16 + (10 * m.nt + 3 if name == "linear_adr" else 0), name
 """)
+
+
+def test_operators_name_the_kernel_that_they_run(fake):
+    run(fake, """
+for shape in SHAPES:
+    for name in OPS:
+        for nm in (4, 12):  # 13 points: beyond the line kernels
+            kernel = nb.Operator(name, mesh(shape, nm)).kernel()
+            assert kernel.startswith("k_line" if nm == 4 else "k_generic"), (shape, name, kernel)
+""")
