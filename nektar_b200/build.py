@@ -25,9 +25,8 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-r
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC"]
 
 SOURCES = ["nkb_setup.cpp", "nkb_ops.cu", "nkb_hex.cu", "nkb_hex_f64.cu", "nkb_hex_f32.cu",
-           "nkb_cg.cu", "nkb_static.cu", "nkb_batch.cu", "nkb_dense.cu", "nkb_gen_f64.cu",
-           "nkb_gen_f32.cu", "nkb_tc.cu", "nkb_sc.cu", "nkb_nccl.cpp",
-           "nkb_geom.cu", "nkb_peak.cu", "nkb_line.cu"]
+           "nkb_cg.cu", "nkb_static.cu", "nkb_batch.cu", "nkb_dense.cu", "nkb_tc.cu", "nkb_sc.cu",
+           "nkb_nccl.cpp", "nkb_geom.cu", "nkb_peak.cu", "nkb_line.cu"]
 SOURCES += ["nkb_line_%s_%s.cu" % (op, p) for op in ("bwd", "ip", "pd", "ipd", "helm", "adr")
             for p in ("f64", "f32")]
 

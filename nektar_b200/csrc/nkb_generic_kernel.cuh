@@ -1,6 +1,5 @@
-// The shape-generic element kernel (one template for all shapes, operators
-// and precisions; sizes at run time or, through SDims, at compile time).
-// Included by nkb_ops.cu and by the compile-time-size instantiation units.
+// The shape-generic element kernel: one template for all shapes, operators
+// and precisions, sizes at run time. It serves the sizes that have no line kernel.
 #pragma once
 
 #include "nkb_generic.cuh"
@@ -25,14 +24,10 @@ enum
 };
 
 // per-element shared memory: x[nc] u[nt] g0 g1 g2 [nt] wa[wsz] wb[wsz]
-template <class D> __host__ __device__ constexpr int ElemSmem(const D &d)
+__host__ __device__ inline int ElemSmem(const Dims &d)
 {
     return (d.nc + 4 * d.nt + 2 * d.wsz + 1) & ~1;
 }
-
-// the kernel's dims object: the runtime Dims, or a compile-time SDims
-template <class D> __device__ __forceinline__ D DimsOf(const Dims &) { return D{}; }
-template <> __device__ __forceinline__ Dims DimsOf<Dims>(const Dims &d) { return d; }
 
 template <typename T> struct GenArgs
 {
@@ -72,11 +67,11 @@ template <typename T> struct GenArgs
     }                                                                                             \
     __syncthreads();
 
-template <int SHAPE, int OP, typename T, class D = Dims> __global__ void k_generic(GenArgs<T> a)
+template <int SHAPE, int OP, typename T> __global__ void k_generic(GenArgs<T> a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *smem       = reinterpret_cast<T *>(smem_raw);
-    const D d     = DimsOf<D>(a.d);
+    const Dims d  = a.d;
     const int es  = ElemSmem(d);
     const long e0 = long(blockIdx.x) * a.epb;
     const int ne  = int(min(long(a.epb), long(a.nelmt) - e0));
@@ -201,11 +196,9 @@ template <int SHAPE, int OP, typename T, class D = Dims> __global__ void k_gener
     }
 }
 
-
-
 // Launch of k_generic for one operator: elements per CTA and threads per CTA
 // from the operator's autotuned launch shape (or the defaults).
-template <int SHAPE, int OP, typename T, class D = Dims>
+template <int SHAPE, int OP, typename T>
 int LaunchGenericT(const nkb_op *op, GenArgs<T> a, cudaStream_t s)
 {
     const int es      = ElemSmem(a.d);
@@ -216,7 +209,7 @@ int LaunchGenericT(const nkb_op *op, GenArgs<T> a, cudaStream_t s)
     const int threads = op->gen_threads > 0 ? op->gen_threads : 128;
     a.epb             = epb;
     const size_t smem = ebyt * epb;
-    auto kern         = k_generic<SHAPE, OP, T, D>;
+    auto kern         = k_generic<SHAPE, OP, T>;
     // raise the dynamic shared-memory limit once per instantiation, before any
     // stream capture can contain this launch
     static size_t s_smem_set = 48 * 1024;
@@ -230,36 +223,6 @@ int LaunchGenericT(const nkb_op *op, GenArgs<T> a, cudaStream_t s)
         kern<<<unsigned(nb), threads, smem, s>>>(a);
     NKB_CUDA_TRY(cudaGetLastError());
     return NKB_OK;
-}
-
-// Prism / Tet Helmholtz with compile-time sizes for the standard point sets
-// and nm = 2..11 (instantiated in nkb_gen_f64.cu / nkb_gen_f32.cu). Returns
-// kNotCovered, with no error set, for anything else.
-constexpr int kNotCovered = 1;
-
-template <int SHAPE, typename T> int LaunchHelmStaticShape(const nkb_op *op, const GenArgs<T> &a, cudaStream_t s)
-{
-    switch (op->nm)
-    {
-#define NKB_HS(N)                                                                                  \
-    case N: return LaunchGenericT<SHAPE, GK_HELM, T, SDims<SHAPE, N>>(op, a, s);
-        NKB_HS(2) NKB_HS(3) NKB_HS(4) NKB_HS(5) NKB_HS(6) NKB_HS(7) NKB_HS(8) NKB_HS(9)
-        NKB_HS(10) NKB_HS(11)
-#undef NKB_HS
-        default: return kNotCovered;
-    }
-}
-
-template <typename T> int LaunchHelmStatic(const nkb_op *op, const GenArgs<T> &a, cudaStream_t s)
-{
-    const int nm = op->nm;
-    if (op->nq[0] != nm + 1)
-        return kNotCovered;
-    if (op->shape == NKB_PRISM && op->nq[1] == nm + 1 && op->nq[2] == nm)
-        return LaunchHelmStaticShape<NKB_PRISM, T>(op, a, s);
-    if (op->shape == NKB_TET && op->nq[1] == nm && op->nq[2] == nm)
-        return LaunchHelmStaticShape<NKB_TET, T>(op, a, s);
-    return kNotCovered;
 }
 
 } // namespace nkb

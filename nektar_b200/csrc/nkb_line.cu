@@ -34,17 +34,12 @@ static int LineDispatch(nkb_op *setup, const nkb_op *op, const LineArgs<T> *a, c
     }
 }
 
-static bool EnvIs(const char *name, const char *value)
-{
-    const char *v = std::getenv(name);
-    return v && std::strcmp(v, value) == 0;
-}
-
 int LineSetup(nkb_op *op)
 {
     const bool helm = op->optype == NKB_HELMHOLTZ || op->optype == NKB_LINEAR_ADR;
     const bool hex  = op->shape == NKB_HEX;
-    if (EnvIs("NKB_KERNEL", "generic") || (helm && !hex && EnvIs("NKB_COL", "0")))
+    const char *kernel = std::getenv("NKB_KERNEL");
+    if (kernel && std::strcmp(kernel, "generic") == 0)
         return NKB_OK;
     int v = 0;
     if (HexVariantRequested(op, &v))

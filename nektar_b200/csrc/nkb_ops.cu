@@ -468,15 +468,6 @@ template <int OP, typename T> static int LaunchGenericShape(const nkb_op *op, Ge
     }
 }
 
-extern template int LaunchHelmStatic<double>(const nkb_op *, const GenArgs<double> &, cudaStream_t);
-extern template int LaunchHelmStatic<float>(const nkb_op *, const GenArgs<float> &, cudaStream_t);
-
-static bool StaticSizes()
-{
-    const char *v = std::getenv("NKB_GENERIC_STATIC");
-    return !(v && std::strcmp(v, "0") == 0);
-}
-
 template <typename T>
 int LaunchGeneric(const nkb_op *op, const T *in, T *o0, T *o1, T *o2, const int *gmap,
                   const double *gsign, cudaStream_t s, const int *skip, const double *lambda)
@@ -528,15 +519,7 @@ int LaunchGeneric3(const nkb_op *op, const T *in, const T *in1, const T *in2, T 
         case NKB_LINEAR_ADR:
             return LaunchGenericShape<GK_ADR, T>(op, a, s);
         default:
-        {
-            if (StaticSizes())
-            {
-                const int rc = LaunchHelmStatic<T>(op, a, s);
-                if (rc != kNotCovered)
-                    return rc;
-            }
             return LaunchGenericShape<GK_HELM, T>(op, a, s);
-        }
     }
 }
 

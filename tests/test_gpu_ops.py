@@ -183,28 +183,11 @@ def test_line_kernel_linear_adr_matches_oracle(shape, nm):
     assert rel_l2(op(x), yo) < TOL64
 
 
-@pytest.mark.parametrize("shape,n,nm", [("prism", 2, 4), ("tet", 2, 5), ("prism", 1, 9), ("tet", 1, 11)])
-def test_static_and_runtime_size_generic_helmholtz_agree(monkeypatch, shape, n, nm):
-    """Prism / Tet Helmholtz with compile-time sizes against the same kernel
-    with run-time sizes."""
-    m = nb.BoxMesh(shape, n, nm, nm + 1, amp=0.05)
-    x = np.random.default_rng(nm).uniform(-1, 1, m.nelmt * m.nc)
-    monkeypatch.setenv("NKB_COL", "0")
-    fast = nb.Operator("helmholtz", m)
-    fast.set_factors(0.7)
-    y_fast = fast(x)  # the switches are read at launch time
-    monkeypatch.setenv("NKB_GENERIC_STATIC", "0")
-    slow = nb.Operator("helmholtz", m)
-    slow.set_factors(0.7)
-    assert rel_l2(y_fast, slow(x)) < 1e-13
-
-
 @pytest.mark.parametrize("shape,n,nm", [("prism", 2, 3), ("prism", 1, 8), ("prism", 1, 11),
                                         ("tet", 2, 4), ("tet", 1, 7), ("tet", 1, 11)])
 @pytest.mark.parametrize("precision,tol", [("fp64", 1e-13), ("fp32", 2e-6)])
-def test_column_and_generic_helmholtz_agree(monkeypatch, shape, n, nm, precision, tol):
-    """Prism / Tet column kernels (k direction in registers) against the
-    shape-generic kernel."""
+def test_line_and_generic_helmholtz_agree(monkeypatch, shape, n, nm, precision, tol):
+    """Prism / Tet line kernels against the shape-generic kernel."""
     import torch
     m = nb.BoxMesh(shape, n, nm, nm + 1, amp=0.05)
     x = np.random.default_rng(nm).uniform(-1, 1, m.nelmt * m.nc)
@@ -218,19 +201,19 @@ def test_column_and_generic_helmholtz_agree(monkeypatch, shape, n, nm, precision
         torch.cuda.synchronize()
         return yd.double().cpu().numpy()
 
-    col = nb.Operator("helmholtz", m, precision=precision)
-    col.set_factors(1.3)
-    y_col = apply(col)  # the switch is read at launch time
-    monkeypatch.setenv("NKB_COL", "0")
+    line = nb.Operator("helmholtz", m, precision=precision)
+    line.set_factors(1.3)
+    monkeypatch.setenv("NKB_KERNEL", "generic")
     gen = nb.Operator("helmholtz", m, precision=precision)
     gen.set_factors(1.3)
-    assert rel_l2(y_col, apply(gen)) < tol
+    assert line.kernel().startswith("k_line") and gen.kernel() == "k_generic"
+    assert rel_l2(apply(line), apply(gen)) < tol
 
 
 @pytest.mark.parametrize("shape", ["prism", "tet"])
-def test_column_kernel_gathered_in_cg(monkeypatch, shape):
-    """The column kernels' gathered form (inside the CG): a block-diagonal
-    system (every local dof its own global dof) solved with the column and
+def test_line_kernel_gathered_in_cg(monkeypatch, shape):
+    """The line kernels' gathered form (inside the CG): a block-diagonal
+    system (every local dof its own global dof) solved with the line and
     with the generic kernels."""
     m = nb.BoxMesh(shape, 2, 5, 6, amp=0.05)
     nloc = m.nelmt * m.nc
@@ -240,7 +223,7 @@ def test_column_kernel_gathered_in_cg(monkeypatch, shape):
     op.set_factors(2.0)
     S = nb.GlobalLinSys([op], gmap, nloc, 0)
     xa, ra = S.solve(b, tol=1e-12)
-    monkeypatch.setenv("NKB_COL", "0")
+    monkeypatch.setenv("NKB_KERNEL", "generic")
     op2 = nb.Operator("helmholtz", m)
     op2.set_factors(2.0)
     S2 = nb.GlobalLinSys([op2], gmap, nloc, 0)
