@@ -130,37 +130,46 @@ def test_device_pointer_path_matches_host_path():
     assert np.array_equal(yd.cpu().numpy(), yh)  # same kernel, same order: bitwise
 
 
+# NKB_HEX_VARIANT's FP64 kernels (None: unset) and the kernel each one runs
+HEX_KERNELS = [None, 0]
+
+
+def _hex_operator(monkeypatch, name, m, variant):
+    if variant is not None:
+        monkeypatch.setenv("NKB_HEX_VARIANT", str(variant))
+    op = nb.Operator(name, m)
+    assert op.kernel().startswith("k_line" if variant is None else "k_hex_helm (TMA")
+    return op
+
+
 @pytest.mark.parametrize("n,nm", [(1, 5), (3, 7), (2, 9), (1, 11), (5, 2)])
-@pytest.mark.parametrize("variant", [0, 1, 2, 3, 4, 6, 7, 8])
+@pytest.mark.parametrize("variant", HEX_KERNELS)
 def test_tuned_and_generic_hex_helmholtz_agree(monkeypatch, n, nm, variant):
-    """Every variant of the tuned Hex kernel (nkb_hex.cu: TMA-staged or
-    streamed geometry, 1-2 elements per CTA, FP64 tensor cores for nq <= 8)
-    against the shape-generic kernel, odd element counts included (partially
-    filled last CTA)."""
+    """The line kernel and the TMA-staged Hex kernel (variant 0) against the
+    shape-generic kernel, odd element counts included (partially filled last
+    CTA of the TMA-staged one)."""
     m = nb.BoxMesh("hex", n, nm, nm + 1, amp=0.05)
     x = np.random.default_rng(nm).uniform(-1, 1, m.nelmt * m.nc)
-    monkeypatch.setenv("NKB_HEX_VARIANT", str(variant))
-    tuned = nb.Operator("helmholtz", m)
+    tuned = _hex_operator(monkeypatch, "helmholtz", m, variant)
     tuned.set_factors(0.3)
     monkeypatch.setenv("NKB_KERNEL", "generic")
     generic = nb.Operator("helmholtz", m)
     generic.set_factors(0.3)
+    assert generic.kernel() == "k_generic"
     assert rel_l2(tuned(x), generic(x)) < 1e-13
 
 
 @pytest.mark.parametrize("n,nm", [(1, 5), (3, 7), (2, 9), (1, 11), (5, 2)])
-@pytest.mark.parametrize("variant", [0, 1, 2, 3, 4, 6, 7, 8])
+@pytest.mark.parametrize("variant", HEX_KERNELS)
 def test_hex_kernel_variants_linear_adr_match_oracle(monkeypatch, n, nm, variant):
-    """LinearADR through every variant of the tuned Hex kernel (its advection
-    mode) against the oracle; a variant without room for the three extra
-    geometry rows falls back to the generic kernel."""
+    """LinearADR through the line kernel and the TMA-staged Hex kernel (its
+    advection mode) against the oracle."""
     m = nb.BoxMesh("hex", n, nm, nm + 1, amp=0.05)
     rng = np.random.default_rng(nm + 100)
     x = rng.uniform(-1, 1, m.nelmt * m.nc)
     vel = rng.uniform(-1, 1, 3 * m.nelmt * m.nt)
     k = m.nelmt * m.nt
-    monkeypatch.setenv("NKB_HEX_VARIANT", str(variant))
-    op = nb.Operator("linear_adr", m)
+    op = _hex_operator(monkeypatch, "linear_adr", m, variant)
     op.set_factors(0.6)
     op.set_varcoeffs(vel[:k], vel[k:2 * k], vel[2 * k:])
     yo = O.linear_adr("hex", nm, m.nq, m.nelmt, _oracle_T(m), m.jac, m.df, 0.6, vel, x, True)
@@ -333,16 +342,15 @@ def test_fp32_linear_adr_matches_oracle(shape):
     assert rel_l2(yd.double().cpu().numpy(), yo) < TOL32
 
 
-@pytest.mark.parametrize("variant", [0, 1, 2, 3, 4, 6, 7, 8])
+@pytest.mark.parametrize("variant", HEX_KERNELS)
 def test_hex_kernel_variants_are_repeatable(monkeypatch, variant):
-    """Repeated applications of every Hex variant to one input give the same
+    """Repeated applications of either Hex kernel to one input give the same
     bits: a race between the warps of an element (a shared-memory store
     landing after another warp's copy) shows up as an occasional wrong
     element, which a one-shot comparison can miss."""
     m = nb.BoxMesh("hex", 16, 7, 8, amp=0.05)
     x = np.random.default_rng(11).uniform(-1, 1, m.nelmt * m.nc)
-    monkeypatch.setenv("NKB_HEX_VARIANT", str(variant))
-    op = nb.Operator("helmholtz", m)
+    op = _hex_operator(monkeypatch, "helmholtz", m, variant)
     op.set_factors(1.0)
     y0 = op(x)
     bad = sum(not np.array_equal(op(x), y0) for _ in range(150))
