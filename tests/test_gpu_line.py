@@ -1,8 +1,8 @@
 """The line kernels (nkb_line_kernel.cuh) against the shape-generic kernels:
 every operator on every shape, at the smallest and largest orders, point counts
 whose shared-memory rows are rotated (4 and 8) and not, over-integration,
-straight-sided and curved geometry, and element counts that leave the last CTA
-partly filled."""
+straight-sided and curved geometry; collections of one element per CTA, of several,
+and of full CTAs with the last one partly filled."""
 import numpy as np
 import pytest
 
@@ -59,6 +59,94 @@ def test_line_and_generic_kernels_agree(monkeypatch, shape, nm, nq, amp, precisi
             x = np.random.default_rng(nq).uniform(-1, 1, line.in_size)
             y, z = _apply(line, x, dtype), _apply(generic, x, dtype)
             assert rel_l2(y, z) < TOL[precision], (name, n, line.kernel())
+
+
+def _full_cta_elements(shape, nq):
+    """A count that fills every CTA, whatever the elements per CTA: more than all
+    threads of the device at one line of points each."""
+    import torch
+    lines = nq * (nq if shape != "tet" else nq - 1)
+    return torch.cuda.get_device_properties(0).multi_processor_count * 2048 // lines + 1
+
+
+def _random_operator(name, shape, nm, nq, nelmt, curved, precision):
+    """Elements whose factors vary from one to the next (and from point to point)."""
+    import torch
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(nelmt)
+    T, q = nb.shape_tables(shape, nm, nq)
+    nt = q[0] * q[1] * q[2]
+    n = nelmt * nt if curved else nelmt
+    rand = lambda *s: torch.rand(*s, generator=gen, dtype=torch.float64, device="cuda") * 2 - 1
+    jac, df = 1 + 0.3 * rand(n), 0.25 * rand(9, n)
+    df[0::4] += 1
+    op = nb.Operator(name, shape=shape, nm=nm, nq=q, nelmt=nelmt, T=T, jac=jac, df=df,
+                     deformed=curved, precision=precision)
+    if name in ("helmholtz", "linear_adr"):
+        op.set_factors(0.7)
+    if name == "linear_adr":
+        vel = rand(3, nelmt * nt)
+        op.set_varcoeffs(*[v.data_ptr() for v in vel])
+    return op
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("nm,nq", [(2, 3), (3, 4), (4, 5), (5, 6), (7, 8), (8, 9), (10, 11), (2, 4),
+                                   (4, 8), (5, 9)])
+@pytest.mark.parametrize("shape", ["hex", "prism", "tet"])
+def test_full_and_partly_filled_ctas(monkeypatch, shape, nm, nq, precision):
+    """Collections beyond one wave, where each CTA takes as many elements as it can:
+    of two consecutive counts at least one leaves the last CTA partly filled. Below
+    it, a collection of half that size, at a few elements per CTA."""
+    import torch
+    dtype = torch.float64 if precision == "fp64" else torch.float32
+    full = _full_cta_elements(shape, nq)
+    monkeypatch.setenv("NKB_GENERIC_TUNE", "0")
+    for k, name in enumerate(OPS):
+        for nelmt in (full + nq, full + nq + 1, full // 3):
+            for curved in (True, False):
+                if name == "bwdtrans" and not curved:
+                    continue  # no geometry
+                args = name, shape, nm, nq, nelmt, curved, precision
+                line = _random_operator(*args)
+                monkeypatch.setenv("NKB_KERNEL", "generic")
+                generic = _random_operator(*args)
+                monkeypatch.delenv("NKB_KERNEL")
+                assert line.kernel().startswith("k_line") and generic.kernel() == "k_generic"
+                x = torch.rand(line.in_size, dtype=dtype, device="cuda") * 2 - 1
+                s = torch.cuda.current_stream().cuda_stream
+                nout = 3 if name == "physderiv" else 1
+                y, z = (torch.full((nout, op.out_size), float("nan"), dtype=dtype, device="cuda")
+                        for op in (line, generic))
+                for op, out in ((line, y), (generic, z)):
+                    op.apply_device(x.data_ptr(), *[o.data_ptr() for o in out], stream=s)
+                d, z = (y.double() - z.double()).view(nout, nelmt, -1), z.double().view(nout, nelmt, -1)
+                # of every element by itself: the largest of 1e4 to 1e5 of them lies
+                # within ten times the bound that holds for all together
+                each = d.square().sum((0, 2)).sqrt() / z.square().sum((0, 2)).mean().sqrt()
+                assert d.norm() < TOL[precision] * z.norm(), args
+                assert each.max() < 10 * TOL[precision], args
+                line.close(), generic.close()
+
+
+@pytest.mark.parametrize("shape,nm,nq", [("hex", 3, 4), ("prism", 5, 6), ("tet", 4, 5), ("tet", 6, 9)])
+def test_gathered_launches_of_full_ctas(monkeypatch, shape, nm, nq):
+    """Three CG iterations of a block-diagonal system with signs and a permuted map,
+    on full CTAs of the line and of the generic kernel."""
+    nelmt = _full_cta_elements(shape, nq) + nq
+    rng = np.random.default_rng(nq)
+    nloc = nelmt * nb.ncoeffs(shape, nm)
+    gmap, sign = rng.permutation(nloc).astype(np.int32), rng.choice([-1.0, 1.0], nloc)
+    b, xs = rng.uniform(-1, 1, nloc), []
+    for kernel in (None, "generic"):
+        if kernel:
+            monkeypatch.setenv("NKB_KERNEL", kernel)
+        op = _random_operator("helmholtz", shape, nm, nq, nelmt, True, "fp64")
+        S = nb.GlobalLinSys([op], gmap, nloc, 0, sign=sign)
+        xs.append(S.solve(b, tol=1e-14, maxit=3, check_interval=3, raise_on_maxit=False)[0])
+    # three iterations magnify the operators' TOL by a few times the ratio of
+    # the largest to the smallest entry of the diagonal (about 1e2)
+    assert np.abs(xs[0]).max() > 0 and rel_l2(*xs) < 1e2 * TOL["fp64"]
 
 
 @pytest.mark.parametrize("shape", ["hex", "prism", "tet"])
