@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 
 namespace nkb
 {
@@ -196,6 +197,14 @@ template <int SHAPE, int OP, typename T> __global__ void k_generic(GenArgs<T> a)
     }
 }
 
+// A kernel's limit is raised to what a block can have, whatever this launch needs:
+// another size's launch, on another thread, must not lower it under this one's.
+inline cudaError_t RaiseSmemLimit(const void *kern, size_t smem)
+{
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                int(std::max<size_t>(smem, 227 * 1024)));
+}
+
 // Launch of k_generic for one operator: elements per CTA and threads per CTA
 // from the operator's autotuned launch shape (or the defaults).
 template <int SHAPE, int OP, typename T>
@@ -210,13 +219,14 @@ int LaunchGenericT(const nkb_op *op, GenArgs<T> a, cudaStream_t s)
     a.epb             = epb;
     const size_t smem = ebyt * epb;
     auto kern         = k_generic<SHAPE, OP, T>;
-    // raise the dynamic shared-memory limit once per instantiation, before any
-    // stream capture can contain this launch
-    static size_t s_smem_set = 48 * 1024;
-    if (smem > s_smem_set)
+    // the dynamic shared-memory limit is raised once per instantiation and device
+    // (a bit each), before any stream capture can contain this launch
+    static std::atomic<unsigned> raised{0};
+    const unsigned bit = op->device < 32 ? 1u << op->device : 0;
+    if (smem > 48 * 1024 && !(raised.load() & bit))
     {
-        NKB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        s_smem_set = smem;
+        NKB_CUDA_TRY(RaiseSmemLimit((const void *)kern, smem));
+        raised.fetch_or(bit);
     }
     const long nb = (long(a.nelmt) + epb - 1) / epb;
     if (nb > 0)

@@ -1194,8 +1194,7 @@ static int HexDiag(const nkb_op *op, const double *geo, double *d_out, cudaStrea
     const int threads = 256;
     const size_t smem =
         (size_t(nm) * nq * nq + size_t(nm) * nm * nq + 2 * size_t(nm) * nm * nm) * sizeof(double);
-    cudaError_t ce = cudaFuncSetAttribute(k_hex_diag, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          int(smem));
+    cudaError_t ce = RaiseSmemLimit((const void *)k_hex_diag, smem);
     if (ce == cudaSuccess && op->nelmt > 0)
     {
         k_hex_diag<<<op->nelmt, threads, smem, s>>>(nm, nq, dtab, geo, op->gstride, op->nelmt,
@@ -1235,7 +1234,7 @@ static int DiagOf(const nkb_op *op, const double *geo, double *d_out, cudaStream
     void (*kern)(GenArgs<double>, int) = op->shape == NKB_HEX     ? k_diag<NKB_HEX, double>
                                     : op->shape == NKB_PRISM ? k_diag<NKB_PRISM, double>
                                                              : k_diag<NKB_TET, double>;
-    NKB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    NKB_CUDA_TRY(RaiseSmemLimit((const void *)kern, smem));
     if (op->nelmt > 0)
         kern<<<op->nelmt, threads, smem, s>>>(a, op->geo_perm);
     NKB_CUDA_TRY(cudaGetLastError());

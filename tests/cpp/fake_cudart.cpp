@@ -7,6 +7,8 @@
 
 #include <cstdlib>
 #include <cstring>
+#include <map>
+#include <utility>
 #include <vector>
 
 namespace
@@ -18,6 +20,9 @@ struct Write
 };
 std::vector<Write> outstanding;
 int early_launches = 0, launches = 0, attribute_queries = 0;
+std::map<std::pair<int, const void *>, size_t> smem_limit; // by device and kernel
+int device             = 0;
+cudaError_t last_error = cudaSuccess;
 long next_handle = 0x1000, allocated = 0;
 
 bool Legacy(cudaStream_t s)
@@ -82,28 +87,43 @@ cudaError_t __cudaPopCallConfiguration(dim3 *g, dim3 *b, size_t *m, void *s)
     *static_cast<void **>(s) = call.stream;
     return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void *, dim3 grid, dim3 block, void **, size_t, cudaStream_t s)
+cudaError_t cudaLaunchKernel(const void *kernel, dim3 grid, dim3 block, void **, size_t smem,
+                             cudaStream_t s)
 {
     if (!grid.x || !grid.y || !grid.z || !block.x)
-        return cudaErrorInvalidConfiguration;
+        return last_error = cudaErrorInvalidConfiguration;
+    const auto limit = smem_limit.find({device, kernel});
+    if (smem > (limit == smem_limit.end() ? 48 * 1024 : limit->second))
+        return last_error = cudaErrorInvalidValue;
     ++launches;
     if (!Legacy(s) && !outstanding.empty())
         ++early_launches;
     return cudaSuccess;
 }
 
-cudaError_t cudaGetDeviceCount(int *n) { return *n = 1, cudaSuccess; }
-cudaError_t cudaGetDevice(int *d) { return *d = 0, cudaSuccess; }
-cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetDeviceCount(int *n) { return *n = 2, cudaSuccess; }
+cudaError_t cudaGetDevice(int *d) { return *d = device, cudaSuccess; }
+cudaError_t cudaSetDevice(int d) { return device = d, cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int)
 {
     ++attribute_queries;
     return *v = 148, cudaSuccess;
 }
 cudaError_t cudaRuntimeGetVersion(int *v) { return *v = CUDART_VERSION, cudaSuccess; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError()
+{
+    const cudaError_t e = last_error;
+    last_error          = cudaSuccess;
+    return e;
+}
 const char *cudaGetErrorString(cudaError_t) { return "fake"; }
-cudaError_t cudaFuncSetAttribute(const void *, cudaFuncAttribute, int) { return cudaSuccess; }
+cudaError_t cudaFuncSetAttribute(const void *kernel, cudaFuncAttribute, int v)
+{
+    if (v > 227 * 1024)
+        return cudaErrorInvalidValue;
+    smem_limit[{device, kernel}] = size_t(v);
+    return cudaSuccess;
+}
 
 cudaError_t cudaMalloc(void **p, size_t n)
 {

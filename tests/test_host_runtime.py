@@ -137,3 +137,18 @@ for shape in SHAPES:
             kernel = nb.Operator(name, mesh(shape, nm)).kernel()
             assert kernel.startswith("k_line" if nm == 4 else "k_generic"), (shape, name, kernel)
 """)
+
+
+def test_shared_memory_is_allowed_on_every_device(fake):
+    """The generic kernels' limit is raised on each device that they run on, and a small
+    operator's launches and diagonal leave it for a large one's."""
+    run(fake, """
+x = np.zeros(1)
+for shape in SHAPES:
+    for device in (0, 1):
+        ops = [nb.Operator("helmholtz", mesh(shape, nm), device=device) for nm in (14, 12)]
+        for op in ops + ops[:1]:
+            op.apply_device(x.ctypes.data, x.ctypes.data)
+            op.helmholtz_diag()
+            op.apply_device(x.ctypes.data, x.ctypes.data)
+""", NKB_GENERIC_TUNE="0")
