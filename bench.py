@@ -462,7 +462,7 @@ def hex_flops(nm, nq):
 
 def operator_roofline(nb, torch, dev, n, p, precision, hbm, iters=20, peaks=None):
     """Element Helmholtz apply on an n^3 curved box at order p (local
-    vectors, autotuned kernel): ms, GB/s of the algorithmic bytes, fraction;
+    vectors): ms, GB/s of the algorithmic bytes, fraction;
     with peaks, TFLOP/s of the algorithmic FLOPs and their fraction of the
     precision's measured rate (FP64: the higher of FMA and tensor-core MMA)."""
     nm = p + 1

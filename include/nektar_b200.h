@@ -278,7 +278,9 @@ int nkb_op_last_kernel_ms(const nkb_op *op, float *ms);
 int nkb_op_check_error(nkb_op *op);
 
 /* Test hook: the number of polls after which a bounded wait inside the
- * operator's kernels gives up (0: at once; negative: the default, 2^24). A
+ * operator's kernels gives up (0: at once; negative: the default, 2^24). Only
+ * the Hex kernels that NKB_HEX_VARIANT requests wait; the line and generic
+ * kernels do not, and the limit has no effect on them. A
  * wait that gives up records NKB_ERR_TIMEOUT and still waits (bounded) for
  * its copy or MMA to complete before the kernel exits. Used by the tests to
  * make the wait run out; no reference counterpart. */

@@ -1,15 +1,26 @@
 // Line kernels: the element operators with one thread per grid line.
 //
-// Every one-dimensional contraction (basis to points, points to basis, the
+// A one-dimensional contraction (basis to points, points to basis, the
 // collocation derivative and its transpose) is done by a thread that loads one
 // whole line of the element into registers, multiplies it by the 1-D table and
 // stores the whole result line. The tables are kernel parameters and every
 // index into them is a compile-time constant, so the n*n multiply-adds of a
 // line cost n loads and n stores of shared memory and no table traffic; a
 // thread that computes one output per dot product (the shape-generic kernel)
-// loads 2n values for n multiply-adds. What bounds the operators is then
-// memory (curved elements) or, for straight-sided ones, the mix of FP64
-// multiply-adds and shared-memory wavefronts, which are about equal at 8 points.
+// loads 2n values for n multiply-adds.
+//
+// That holds for every stage of a hexahedron, every derivative, and the first
+// direction of the collapsed shapes (and a prism's second). Their third
+// direction's table depends on (p, q): a thread keeps one column (or row) of it
+// in registers, walks the CTA's elements, and takes one shared load per
+// multiply-add. A tetrahedron's second direction depends on p, which differs
+// between a warp's lanes: its table entries are global loads (L1), one per
+// multiply-add.
+//
+// What bounds the operators: HBM for curved hexahedra in FP64 (Helmholtz at 0.72 of
+// the copy rate in long runs under the power cap, 0.82 in short ones, PhysDeriv
+// 0.81), instruction issue in FP32 (79 %), the
+// L1/shared pipe for prisms and tetrahedra (70 to 81 %).
 //
 // Directions. A kernel has a register direction (0) and two lane directions
 // (1, and 2 fastest). Hexahedra, and PhysDeriv on every shape, take the mesh's
@@ -175,7 +186,10 @@ constexpr int LineDealt(const LineCounts &h, int shift, int epb, int banks, int 
     return (most < phases ? most : phases) + over;
 }
 
-// about the accesses of the Helmholtz operator per line and direction
+// About the accesses of the Helmholtz operator per line and direction. The other
+// operators' layouts follow them too: with equal weights, FP64 BwdTrans, IProduct,
+// IProductWRTDerivBase and PhysDeriv of 3 to 10 modes took 0.92 to 1.05 of the
+// time, within 1 % at 123 of 144 sizes.
 constexpr int LineCost(int r, int b, int c, int k0, int k1, int k2)
 {
     return 8 * k0 * r + 7 * k1 * b + 6 * k2 * c;
@@ -285,12 +299,13 @@ template <int SHAPE, int NM, int NQ, int OP, typename T> struct LineDims
     static constexpr int PS = LAY.ps, CUBE = LAY.cube;
     static constexpr bool DEALT = DEAL && !LAY.rotate && EPB < 31;
     static_assert(EPB * CUBE < 65536, "line offsets have 16 bits");
-    // register budget per thread: the lowest that spills (next to) nothing. Warps
-    // in flight hide the barriers and the shared-memory latency: at 80 instead of
-    // 128 registers the FP64 Helmholtz operator took 87 instead of 118 us (hex, 8
-    // modes x 7140), 103 instead of 143 (9 x 5172), 115 instead of 184 (tet, 8 x
-    // 10241); FP32 at 48 instead of 64 gained 0-25 %
-        // (PhysDeriv's FP64 chain rule and LinearADR's extra rows take more)
+    // register budget per thread: the lowest that spills next to nothing (49 of the
+    // 630 instantiations spill, 4 to 92 bytes; PhysDeriv's FP64 chain rule and
+    // LinearADR's extra rows take more). Warps in flight hide the barriers and the
+    // shared-memory latency: at 80 instead of 128 registers the FP64 Helmholtz
+    // operator took 87 instead of 118 us (hex, 8 modes x 7140), 103 instead of 143
+    // (9 x 5172), 115 instead of 184 (tet, 8 x 10241); FP32 at 48 instead of 64
+    // gained 0-25 %
     static constexpr int REGS =
         sizeof(T) == 8 ? (K0 <= (OP == LN_ADR ? 9 : 10) ? 80 : 96)
                        : (OP == LN_PD && SHAPE == NKB_TET ? 56 : (K0 <= 9 ? 48 : 64));
@@ -469,7 +484,11 @@ __global__ void __launch_bounds__(LineDims<SHAPE, NM, NQ, OP, T>::TH,
 
     // the CTA's points in the arrays' order, fn(element, point, i, j, k): a point's
     // indices are worked out once for all elements, or, with few elements, per
-    // point so that several are in flight
+    // point so that several are in flight. Unrolled, several points' loads are in
+    // flight at once: without it FP64 IProduct took 1.09 to 1.51 times as long
+    // (prisms and tets of 3 to 10 modes), IProductWRTDerivBase, whose points take
+    // three loads each, 0.95 to 1.13 (prisms) and 0.97 to 1.21 (tets) and BwdTrans,
+    // which only stores, 0.93 to 1.04
     auto each_point = [&](auto fn) {
         if constexpr (L::EPB >= 2)
         {

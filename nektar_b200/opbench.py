@@ -60,10 +60,13 @@ def main():
     e1.record(s)
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1) / a.iters
-    ncomp = {"helmholtz": 7, "linear_adr": 10, "physderiv": 9, "iproduct_deriv": 9,
+    # the Jacobian, metric or derivative factors of every point, or of a straight-sided
+    # element; velocities vary from point to point on any mesh
+    ncomp = {"helmholtz": 7, "linear_adr": 7, "physderiv": 9, "iproduct_deriv": 9,
              "iproduct": 1, "bwdtrans": 0}[a.op]
     esz = 8 if a.precision == "fp64" else 4
-    byts = m.nelmt * esz * (ncomp * m.nt + (op.in_size + len(outs) * op.out_size) / m.nelmt)
+    geometry = ncomp * (m.nt if m.deformed else 1) + (3 * m.nt if a.op == "linear_adr" else 0)
+    byts = m.nelmt * esz * (geometry + (op.in_size + len(outs) * op.out_size) / m.nelmt)
     print(json.dumps({"op": a.op, "shape": a.shape, "n": a.n, "P": a.p, "nelmt": m.nelmt,
                       "precision": a.precision, "kernel": op.kernel(), "ms": ms,
                       "GB_s": byts / ms / 1e6, "GDOF_s": m.nelmt * m.nc / ms / 1e6}))
